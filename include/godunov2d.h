@@ -228,7 +228,10 @@ int gd2d_calc_diff_term(gd2d_handle *h, int32_t icase, double *diff);
 int gd2d_autotune(gd2d_handle *h, int32_t steps_per_trial, gd2d_launch *chosen);
 
 /* Device time of the kernels of the last propagate call (CUDA events on the
- * handle's stream): total ms and ms of the fused cell kernel. */
+ * handle's stream): total ms and ms of the fused cell kernel.  The cell
+ * kernel is timed on one step of a call (the last one of the call's last
+ * step graph, or of the call); of calls of one step, the first and every
+ * 32nd after it are timed and the others report the last one timed. */
 int gd2d_last_timing(gd2d_handle *h, double *total_ms, double *cell_kernel_ms, int64_t *launches);
 
 int gd2d_destroy(gd2d_handle *h);
