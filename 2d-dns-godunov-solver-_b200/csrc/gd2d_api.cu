@@ -339,6 +339,15 @@ DevCase make_devcase(const gd2d_params &p, double maxEdge) {
     d.suth_ref = 1.4792e-6 * std::sqrt(p.T_ref) / (1.0 + 116.0 / p.T_ref);
     d.gamma_over_Pr = p.Gamma / p.Pr;
     d.maxEdge = maxEdge;
+    d.face.gamma = p.Gamma;
+    d.face.gm1 = p.Gamma - 1.0;
+    d.face.rgm1 = 1.0 / d.face.gm1;
+    d.face.g2 = 2.0 * (p.Gamma - 1.0) / (p.Gamma + 1.0);
+    d.face.ksi = p.ksi;
+    d.face.venkat_K = p.venkat_K;
+    d.face.limiter = p.limiter;
+    d.rR = 1.0 / d.R;
+    d.rsuth = 1.0 / d.suth_ref;
     d.tgv_U0 = p.tgv_U0;
     d.tgv_P0 = p.tgv_P0;
     d.tgv_L = p.tgv_L;
@@ -359,6 +368,25 @@ DevCase make_devcase(const gd2d_params &p, double maxEdge) {
     d.art_visc = p.art_viscosity;
     d.limiter = p.limiter;
     return d;
+}
+
+// Whether a case's constants and cell geometry are in the range for which the
+// straight-line quotients of face_exact.cuh round correctly (any case in
+// physical units is); if not, its cells are evaluated by the plain formulas.
+bool exact_rows_case(const DevCase &d, const gd2d_mesh_view &mv) {
+    auto in = [](double x, double lo, double hi) { return x >= lo && x <= hi; };  // false for NaN
+    // divisors with an all-ones significand are the method's exception
+    auto divisor = [&](double x) {
+        uint64_t b;
+        std::memcpy(&b, &x, sizeof b);
+        return in(x, 1e-20, 1e20) && (b & 0xffffffffu) != 0xffffffffu;
+    };
+    if (!divisor(d.face.gm1) || !divisor(d.R) || !in(d.gamma, 1.01, 100.0)) return false;
+    if (d.visc_model == VISC_SUTHERLAND && !divisor(d.suth_ref)) return false;
+    if (!in(d.venkat_K, 0.0, 1e6) || !in(d.ksi, 0.0, 1e20)) return false;
+    for (int64_t i = 0; i < mv.n_cells; ++i)
+        if (!divisor(mv.cell_areas[i]) || !divisor(mv.HX[i])) return false;
+    return true;
 }
 
 template <class T>
@@ -437,9 +465,8 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
     }
     h->lc.persistent = h->launch.persistent;
     // register budget of the cell kernel, measured best on the 2.09M-cell
-    // viscous cylinder: 3 blocks/SM for the FP64 kernels (the tile-face
-    // kernel holds its next face record through the current face), 4 for
-    // the mixed kernels
+    // viscous cylinder: 3 blocks/SM for the FP64 kernels (the tile loop of a
+    // small mesh: see below), 4 for the mixed kernels
     h->lc.min_blocks = h->launch.min_blocks ? h->launch.min_blocks : (h->mixed ? 4 : 3);
     if (h->lc.min_blocks < 2 || h->lc.min_blocks > 4) {
         delete h;
@@ -656,6 +683,7 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
         d.group_begin = ngroups;
         ngroups += (d.tile_end - d.tile_begin + kGroupTiles - 1) / kGroupTiles;
         d.group_end = ngroups;
+        d.face.exact_rows = exact_rows_case(d, mv) ? 1 : 0;
         for (int64_t t = d.tile_begin; t < d.tile_end; ++t) tile_case[t] = c;
         const int64_t node_end = (c + 1 < n_cases) ? h->cases[c + 1].node_off : Nn;
         for (int64_t j = hc.node_off; j < node_end; ++j) node_case[j] = c;
@@ -663,6 +691,35 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
     }
     h->tile_case_h = tile_case;
     h->ngroups = ngroups;
+
+    // each cell's nodes in edge order, if the edges of every cell are a
+    // closed walk in face order (as the reference's meshes list them): the
+    // gradient passes then gather a node once instead of once per edge.  An
+    // edge's two nodes enter symmetrically, so they may be listed either way.
+    std::vector<int4> cn;
+    if (h->visc) {
+        cn.assign(Nc, make_int4(0, 0, 0, 0));
+        bool closed = true;
+        for (int c = 0; c < n_cases && closed; ++c) {
+            const HostCase &hc = h->cases[c];
+            for (int64_t g = hc.cell_off; g < hc.cell_off + hc.nc && closed; ++g) {
+                const int nf = nbr[g].w != kAbsent ? 4 : 3;
+                int n[4] = {0, 0, 0, 0};
+                for (int k = 0; k < nf; ++k) {
+                    // node k is the one that edges k - 1 and k share
+                    const int2 p = c2n[(size_t)((k + nf - 1) % nf) * Nc + g], q = c2n[(size_t)k * Nc + g];
+                    n[k] = (q.x == p.x || q.x == p.y) ? q.x : q.y;
+                }
+                for (int k = 0; k < nf; ++k) {
+                    const int2 q = c2n[(size_t)k * Nc + g];
+                    const int a = n[k], b = n[(k + 1) % nf];
+                    closed &= (q.x == a && q.y == b) || (q.x == b && q.y == a);
+                }
+                cn[g] = make_int4(n[0], n[1], n[2], n[3]);
+            }
+        }
+        if (!closed) cn.clear();
+    }
 
     // face list for the face-loop variants: each interior face once (from its
     // lower-indexed cell), boundary faces once; greedy edge colouring so that
@@ -748,6 +805,7 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
             return true;
         };
         tf_off.assign(ntiles + 1, 0);
+        tf_rec.reserve((size_t)nfmax * Nc * 11 / 20);
         for (int64_t t = 0; t < ntiles; ++t) {
             for (int la = 0; la < block; ++la) {
                 const int64_t g = t * block + la;
@@ -774,6 +832,7 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
                     tf_rec.push_back(make_int4(code, pack_tile_face(la, k, lbp, kb, quad), code_k(dn[g], k),
                                                code_k(up[g], k)));
                     if (h->quads) tf_q.push_back(make_int2(code_k(dn2[g], k), code_k(up2[g], k)));
+                    if (!h->mixed) continue;  // the FP64 kernel reads the per-cell planes
                     const size_t o = (size_t)k * Nc + g;
                     if (h->visc) tf_e.push_back(c2n[o]);
                     tf_nx.push_back(gnx[o]);
@@ -799,7 +858,7 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
     m.Nc = Nc; m.Nn = Nn; m.ncases = n_cases; m.nfmax = nfmax; m.cluster_w = W; m.unit_weights = unit ? 1 : 0;
     m.ntiles = ntiles;
     int4 *d_nbr, *d_dn, *d_up, *d_dn2 = nullptr, *d_up2 = nullptr;
-    int2 *d_c2n;
+    int2 *d_c2n = nullptr;
     double *d_nx, *d_ny, *d_len, *d_rarea, *d_area, *d_hx, *d_charlen, *d_xn = nullptr, *d_yn = nullptr, *d_wt = nullptr;
     double2 *d_mid = nullptr;
     int32_t *d_cl, *d_tc, *d_nc = nullptr;
@@ -829,7 +888,15 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
     ALLOC(d_dn, Nc); UPLOAD(d_dn, dn);
     ALLOC(d_up, Nc); UPLOAD(d_up, up);
     if (h->quads) { ALLOC(d_dn2, Nc); UPLOAD(d_dn2, dn2); ALLOC(d_up2, Nc); UPLOAD(d_up2, up2); }
-    ALLOC(d_c2n, (size_t)nfmax * Nc); UPLOAD(d_c2n, c2n);
+    // (with cn the FP64 kernels read c2n for the analytic ghost state only)
+    if (h->mixed || h->tgv || cn.empty()) { ALLOC(d_c2n, (size_t)nfmax * Nc); UPLOAD(d_c2n, c2n); }
+    if (!cn.empty()) {
+        int4 *d_cn;
+        ALLOC(d_cn, Nc); UPLOAD(d_cn, cn);
+        m.cn = d_cn;
+    }
+    m.exact_rows = 1;
+    for (const DevCase &d : h->hcases) m.exact_rows &= d.face.exact_rows;
     if (!h->mixed) {
         ALLOC(d_nx, (size_t)nfmax * Nc); UPLOAD(d_nx, gnx);
         ALLOC(d_ny, (size_t)nfmax * Nc); UPLOAD(d_ny, gny);
@@ -838,6 +905,20 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
         ALLOC(d_area, Nc); UPLOAD(d_area, area);
         ALLOC(d_hx, Nc); UPLOAD(d_hx, hx);
         ALLOC(d_charlen, Nc); UPLOAD(d_charlen, charlen);
+        if (h->loop == GD2D_LOOP_TILE_FACES) {
+            std::vector<double> eh(Nc, 0.0);
+            for (int c = 0; c < n_cases; ++c) {
+                const HostCase &hc = h->cases[c];
+                if (params[c].limiter != GD2D_LIM_VENKAT) continue;
+                for (int64_t g = hc.cell_off; g < hc.cell_off + hc.nc; ++g) {
+                    const double K = params[c].venkat_K * hx[g];
+                    eh[g] = 0.5 * (K * K * K);
+                }
+            }
+            double *d_eh;
+            ALLOC(d_eh, Nc); UPLOAD(d_eh, eh);
+            m.eh = d_eh;
+        }
     } else {
         d_nx = d_ny = d_len = d_rarea = d_area = d_hx = d_charlen = nullptr;
         auto to_f = [](const std::vector<double> &v) {
@@ -903,7 +984,7 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
         ALLOC(d_tfo, tf_off.size()); UPLOAD(d_tfo, tf_off);
         ALLOC(d_tfr, tf_rec.size()); UPLOAD(d_tfr, tf_rec);
         if (h->quads) { ALLOC(d_tfq, tf_q.size()); UPLOAD(d_tfq, tf_q); }
-        if (h->visc) {
+        if (h->mixed && h->visc) {
             int2 *d_tfe;
             ALLOC(d_tfe, tf_e.size()); UPLOAD(d_tfe, tf_e);
             m.tf_e = d_tfe;
@@ -964,6 +1045,16 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
     {
         int dev_sms = 148;
         cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, h->device);
+        if (!h->launch.min_blocks && !h->mixed && h->loop == GD2D_LOOP_TILE_FACES) {
+            // FP64 tile loop: the 2-block budget (no spills, a tile in less
+            // time) where it takes no more waves of blocks than the 3-block
+            // one.  us a step, 2 / 3 blocks: square 80 tiles 17.1 / 17.9,
+            // Taylor-Green 512 36.8 / 38.3, Roe square 556 37.0 / 41.9; more
+            // waves: quads 352 51.0 / 47.4, square 704 33.8 / 32.7, cylinder
+            // 2044 123 / 116, 8172 440 / 411
+            const int64_t per = dev_sms * (256 / block), w2 = (ntiles + 2 * per - 1) / (2 * per);
+            h->lc.min_blocks = w2 <= (ntiles + 3 * per - 1) / (3 * per) ? 2 : 3;
+        }
         h->lc.grid = dev_sms * h->lc.min_blocks * (256 / block);
     }
     h->history.assign(n_cases, {});

@@ -40,10 +40,24 @@ enum PartSlot {
     P_BAD = 13
 };
 
+// The constants of a case's face formulas, which the tile kernels copy to
+// shared memory: read through the case record they were reloaded from global
+// memory for every face.
+struct FaceCase {
+    double gamma;
+    double gm1, rgm1;   // gamma - 1; 1/(gamma - 1) correctly rounded
+    double g2;          // 2 (gamma - 1) / (gamma + 1)
+    double ksi, venkat_K;
+    int32_t limiter;
+    int32_t exact_rows; // the case's constants and geometry are in the range of face_exact.cuh
+};
+
 // Per-case constants (read-only on the device).
 struct DevCase {
+    FaceCase face;
     double gamma, R, CFL, dt_fixed, beta, ksi, venkat_K;
     double mu_ref, suth_ref, gamma_over_Pr, maxEdge;
+    double rR, rsuth;                 // 1/R, 1/suth_ref correctly rounded
     double tgv_U0, tgv_P0, tgv_L, tgv_mu;
     double rho_min, rho_max;          // densityConstrained clamp
     double bc_rho[kMaxBC], bc_u[kMaxBC], bc_v[kMaxBC], bc_p[kMaxBC], bc_Tw[kMaxBC];
@@ -84,12 +98,16 @@ struct DevMesh {
     int32_t ncases, nfmax;   // nfmax: 3 or 4
     int32_t cluster_w;       // ELL width of the cluster lists
     int32_t unit_weights;    // all node_stencils on live slots are 1.0
+    int32_t exact_rows;      // every case has FaceCase::exact_rows
     int64_t ntiles;
     const int4 *nbr;
     const int4 *dn, *up, *dn2, *up2;     // dn2/up2 only with quads
     const int2 *c2n;                     // [nfmax][Nc] edge node pairs
+    const int4 *cn;                      // [Nc] (viscous) a cell's nodes in edge order: edge k joins nodes k and
+                                         // k + 1 (the last one and the first); NULL if some cell's edges do not
     const double *nx, *ny, *len;         // [nfmax][Nc]
     const double *rarea, *area, *hx, *charlen;
+    const double *eh;                    // (FP64 tile loop) half of (venkat_K hx)^3, zero for other limiters
     const double2 *mid;                  // TGV only
     const double *xnode, *ynode;         // TGV only
     const int32_t *cl;                   // [cluster_w][Nn], -1 = empty

@@ -20,7 +20,7 @@ namespace {
 
 template <int FLUX, bool VISC, bool QUAD, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_cell_step_mixed(const DevMesh m, const DevState s) {
-    __shared__ double s_red[kPartFields * 256];
+    __shared__ double s_red[8 * kPartials];
     const int par = *s.parity;
     const float4 *__restrict__ pin = s.primf + (int64_t)par * m.Nc;
     float4 *__restrict__ pout = s.primf + (int64_t)(par ^ 1) * m.Nc;
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(256, GD2D_NODE_MINB_MIXED) k_grad1_nodes_mixed
 // U holds FP64 primitives on entry: conservatives (utilsFVM2dp.jl:4-17) and
 // the FP32 primitives are written, with the first dt's reductions.
 __global__ void __launch_bounds__(256) k_init_state_mixed(const DevMesh m, const DevState s, int64_t t0, int64_t t1) {
-    __shared__ double s_red[kPartFields * 256];
+    __shared__ double s_red[8 * kPartials];
     const int par = *s.parity;
     float4 *__restrict__ pout = s.primf + (int64_t)par * m.Nc;
     for (int64_t tile = t0 + blockIdx.x; tile < t1; tile += gridDim.x) {

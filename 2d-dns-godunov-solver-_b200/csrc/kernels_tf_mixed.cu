@@ -28,9 +28,7 @@ __global__ void __launch_bounds__(256, MINB) k_cell_step_tf_mixed(const DevMesh 
     // slots, which the step reduction reuses once they have been consumed;
     // declared as double4 for its 32-byte alignment (float4 views need 16)
     constexpr int kTileBytes = (1 + NS * (VISC ? 2 : 1)) * 256 * 16;
-    constexpr int kRedBytes = kPartFields * 256 * 8;
-    constexpr int kBufBytes = kTileBytes > kRedBytes ? kTileBytes : kRedBytes;
-    __shared__ double4 s_buf[kBufBytes / 32];
+    __shared__ double4 s_buf[kTileBytes / 32];
     __shared__ float s_hx[256];
     float4 *const s_prim = reinterpret_cast<float4 *>(s_buf);
     float4 (*const s_flux)[256] = reinterpret_cast<float4 (*)[256]>(s_prim + 256);

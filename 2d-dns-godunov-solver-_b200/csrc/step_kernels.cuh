@@ -12,6 +12,7 @@
 #include <math.h>
 
 #include "gd2d_internal.h"
+#include "face_exact.cuh"
 #include "physics.cuh"
 
 // Register budget of the node-side passes, as resident 256-thread blocks per SM.
@@ -180,45 +181,84 @@ __device__ __forceinline__ double *part_at(const DevMesh &m, const DevState &s, 
     return FIELD_MAJOR ? s.part + (int64_t)f * m.ntiles + q : s.part + q * kPartials + f;
 }
 
-// The tile's reduction record.  With ALIASED, the staging buffer `red`
-// overlays buffers the block used for the tile, so a barrier retires them
-// first; a buffer of the block's own needs none.  Each field is folded in a
-// fixed order: two shuffle levels over groups of four lanes (so a quarter
-// of the values go through shared memory: `red` holds kPartFields rows of
-// blockDim/4), then blockDim/16 threads a field (224 of 256) fold four
-// values each and a fixed shuffle tree joins them -- eight dependent levels
-// in all.  The record is written by each field group's first thread.
-// Nothing more happens at the tile's end: the next node pass folds the
-// records (fold_field), so no tile waits for a fence or an atomic.  The
-// last barrier retires `red` for the next tile of a persistent block.
+// Largest key of a warp: doubles mapped to unsigned 64-bit keys in their
+// order, the high words' maximum first, then the low words' among its owners
+// (two instructions of the warp's reduction unit in place of five levels of
+// 64-bit shuffles and compares).  `sign` -1 maps the reverse order, for a
+// minimum.  NaN takes the key 0, so that it is passed over as fmax and fmin
+// do; a warp of nothing but NaN gives `none`.
+template <int SIGN>
+__device__ __forceinline__ double warp_extreme(double x, double none) {
+    const int h = hi_word(x);
+    const unsigned flip = (unsigned)(h >> 31) | 0x80000000u;  // all bits of a negative number, the sign of others
+    unsigned kh = (unsigned)h ^ flip, kl = lo_word(x) ^ (unsigned)(h >> 31);
+    if (SIGN < 0) { kh = ~kh; kl = ~kl; }
+    if (x != x) kh = kl = 0u;
+    const unsigned mh = __reduce_max_sync(0xffffffffu, kh);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, kh == mh ? kl : 0u);
+    if (mh == 0u && ml == 0u) return none;
+    unsigned rh = mh, rl = ml;
+    if (SIGN < 0) { rh = ~rh; rl = ~rl; }
+    const unsigned back = (rh >> 31) ? 0x80000000u : 0xffffffffu;
+    return __hiloint2double((int)(rh ^ back), (int)(rl ^ ((rh >> 31) ? 0u : 0xffffffffu)));
+}
+
+// One warp's share of the tile's reduction record: its 32 cells' values
+// folded in a fixed order into 14 doubles of shared memory.  The eight sums
+// of four-component fields are halved between lane pairs at distances 16, 8
+// and 4 (each lane passes on the half it does not keep) and folded over the
+// last four lanes, so that eight full sums take nine exchanges instead of
+// forty.
+__device__ __forceinline__ void warp_record(const Part &p, double *out) {
+    const int lane = threadIdx.x & 31;
+    double v[8] = {p.res[0], p.res[1], p.res[2], p.res[3], p.tot[0], p.tot[1], p.tot[2], p.tot[3]};
+#pragma unroll
+    for (int half = 4, off = 16; half > 0; half >>= 1, off >>= 1) {
+        const bool up = (lane & off) != 0;
+#pragma unroll
+        for (int i = 0; i < half; ++i) {
+            const double send = up ? v[i] : v[i + half], keep = up ? v[i + half] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+        }
+    }
+    double x = v[0], ek = p.ek;
+    x = x + __shfl_xor_sync(0xffffffffu, x, 2);
+    x = x + __shfl_xor_sync(0xffffffffu, x, 1);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) ek = ek + __shfl_xor_sync(0xffffffffu, ek, off);
+    // lane 4 q of the warp holds the sum of field q (its three kept halves)
+    const double vmax = warp_extreme<1>(p.vmax, 0.0), rmin = warp_extreme<-1>(p.rmin, INFINITY);
+    const double rhomin = warp_extreme<-1>(p.rhomin, INFINITY), rhomax = warp_extreme<1>(p.rhomax, -INFINITY);
+    const double bad = __any_sync(0xffffffffu, p.bad > 0.0) ? 1.0 : 0.0;
+    if ((lane & 3) == 0) out[lane >> 2] = x;
+    if (lane == 1) {
+        out[P_EK] = ek; out[P_VMAX] = vmax; out[P_RMIN] = rmin;
+        out[P_RHOMIN] = rhomin; out[P_RHOMAX] = rhomax; out[P_BAD] = bad;
+    }
+}
+// The tile's record from its warps' shares (kPartials doubles each), field f
+// by the caller's thread.
+template <bool FIELD_MAJOR>
+__device__ __forceinline__ void fold_warps(const DevMesh &m, const DevState &s, int64_t tile, int f,
+                                           const double *shares, int nwarps) {
+    double x = shares[f];
+    for (int w = 1; w < nwarps; ++w) x = part_op(f, x, shares[w * kPartials + f]);
+    *part_at<FIELD_MAJOR>(m, s, tile, f) = x;
+}
+
+// The tile's reduction record: every warp's share in shared memory (`shares`
+// holds kPartials doubles a warp), folded by the first threads.  With
+// ALIASED, `shares` overlays buffers the block used for the tile, so a
+// barrier retires them first.  Nothing more happens at the tile's end: the
+// next node pass folds the records (fold_field), so no tile waits for a
+// fence or an atomic.  The last barrier retires `shares`.
 template <bool FIELD_MAJOR, bool ALIASED>
 __device__ __forceinline__ void tile_record(const DevMesh &m, const DevState &s, int64_t tile, const Part &p,
-                                            double *red) {
-    const int B = blockDim.x, t = threadIdx.x, lane = t & 31;
-    const int R = B >> 2;    // values per field after the lane folds
-    const int tpf = B >> 4;  // threads per field (4 values each); B is 128 or 256
+                                            double *shares) {
     if (ALIASED) __syncthreads();
-    const double v[kPartFields] = {p.res[0], p.res[1], p.res[2], p.res[3], p.tot[0], p.tot[1], p.tot[2],
-                                   p.tot[3], p.ek, p.vmax, p.rmin, p.rhomin, p.rhomax, p.bad};
-#pragma unroll
-    for (int f = 0; f < kPartFields; ++f) {
-        double x = v[f];
-        x = part_op(f, x, __shfl_down_sync(0xffffffffu, x, 1));
-        x = part_op(f, x, __shfl_down_sync(0xffffffffu, x, 2));
-        if ((lane & 3) == 0) red[f * R + (t >> 2)] = x;
-    }
+    warp_record(p, shares + (threadIdx.x >> 5) * kPartials);
     __syncthreads();
-    const int f = t / tpf, i = t - f * tpf;
-    if (f < kPartFields) {
-        const double *row = red + f * R + i;
-        double x = part_op(f, part_op(f, row[0], row[tpf]), part_op(f, row[2 * tpf], row[3 * tpf]));
-        // a group's lanes are consecutive within one warp (tpf <= 16); the
-        // lanes of this warp below thread kPartFields * tpf take part
-        const int lim = kPartFields * tpf - (t & ~31);
-        const unsigned mask = lim >= 32 ? 0xffffffffu : ((1u << lim) - 1u);
-        for (int off = tpf >> 1; off > 0; off >>= 1) x = part_op(f, x, __shfl_down_sync(mask, x, off, tpf));
-        if (i == 0) *part_at<FIELD_MAJOR>(m, s, tile, f) = x;
-    }
+    if (threadIdx.x < kPartFields) fold_warps<FIELD_MAJOR>(m, s, tile, threadIdx.x, shares, blockDim.x >> 5);
     __syncthreads();
 }
 
@@ -287,15 +327,20 @@ __device__ __forceinline__ void fold_block(const DevMesh &m, const DevState &s, 
 
 // --------------------------------------------------------- MUSCL + flux
 
-// computeInterfaceSlope, computeslope2d.jl:3-136, for face k of cell g with
-// its operands already fetched: neighbour code nbk (cell id or -(bc slot+1)),
-// the neighbour's primitives r and HX (interior faces), the face geometry.
+// computeInterfaceSlope, computeslope2d.jl:3-136, for face k of cell g as it
+// stands in physics.cuh, all operands read from memory: the faces whose
+// operands face_flux_exact does not cover.  nbk: neighbour cell or
+// -(bc slot+1).
 template <int FLUX, bool QUAD>
-__device__ __forceinline__ void face_flux_at(const DevMesh &m, const DevCase &P, const double4 *__restrict__ nodeP,
-                                             int64_t g, int k, int nbk, int dnk, int upk, int dn2k, int up2k,
-                                             bool is_quad, const double *uL, const double4 &r, double hx_own,
-                                             double hxR, double side, double nx, double ny, double t, double g2,
-                                             double *f) {
+__device__ __forceinline__ void face_flux_plain(const DevMesh &m, const DevCase &P, const double4 *__restrict__ pin,
+                                                const double4 *__restrict__ nodeP, int64_t g, int k, int nbk, int dnk,
+                                                int upk, int dn2k, int up2k, bool is_quad, const double *t,
+                                                double *f) {
+    const int64_t og = (int64_t)k * m.Nc + g;
+    const double side = m.len[og], nx = m.nx[og], ny = m.ny[og];
+    const double4 own = pin[g];
+    const double uL[4] = {own.x, own.y, own.z, own.w};
+    double hx_own = m.hx[g], hxR = hx_own;
     double uR[4], uUp[4], uDn[4];
     if (nbk >= 0) {
         if (QUAD && is_quad) {
@@ -309,11 +354,12 @@ __device__ __forceinline__ void face_flux_at(const DevMesh &m, const DevCase &P,
             uUp[0] = a.x; uUp[1] = a.y; uUp[2] = a.z; uUp[3] = a.w;
             uDn[0] = b.x; uDn[1] = b.y; uDn[2] = b.z; uDn[3] = b.w;
         }
+        const double4 r = pin[nbk];
         uR[0] = r.x; uR[1] = r.y; uR[2] = r.z; uR[3] = r.w;
+        hxR = m.hx[nbk];
     } else {
-        bc_ghost<double>(P, m, -nbk - 1, g, k, uL, nx, ny, t, uR);
+        bc_ghost<double>(P, m, -nbk - 1, g, k, uL, nx, ny, *t, uR);
         for (int v = 0; v < 4; ++v) { uDn[v] = uL[v]; uUp[v] = uR[v]; }
-        hxR = hx_own;
     }
     double UpL[4], UpR[4];
     if (P.limiter == LIM_VENKAT) {
@@ -335,7 +381,57 @@ __device__ __forceinline__ void face_flux_at(const DevMesh &m, const DevCase &P,
             UpR[v] = uR[v] - 0.5 * limiter(lk, uR[v] - uL[v], uUp[v] - uR[v], ksi);
         }
     }
-    face_flux_fn<FLUX, double>(UpR, UpL, nx, ny, side, P.gamma, g2, f);
+    face_flux_fn<FLUX, double>(UpR, UpL, nx, ny, side, P.gamma, P.face.g2, f);
+}
+
+// Half of a cell's (K HX)^3, the Venkatakrishnan limiter's scale.
+__device__ __forceinline__ double venkat_half(const FaceCase &P, double hx) {
+    const double K = P.venkat_K * hx;
+    return 0.5 * (K * K * K);
+}
+
+// The same face from operands in registers: the cell's primitives uL, the
+// neighbour's r, the up and down node values a and b (quads: averaged), the
+// face geometry, and with the Venkatakrishnan limiter the two cells' eh =
+// venkat_half.  Straight-line arithmetic (face_exact.cuh); the rare face with
+// an operand out of its range is done over from memory by face_flux_plain
+// (its pointer is made opaque to the compiler, which would otherwise hold
+// every operand in registers across the fast path).
+template <int FLUX, bool QUAD>
+__device__ __forceinline__ void face_flux_at(const DevMesh &m, const DevCase &P, const FaceCase &K,
+                                             const double4 *__restrict__ pin, const double4 *__restrict__ nodeP,
+                                             int64_t g, int k, int nbk, int dnk, int upk, int dn2k, int up2k,
+                                             bool is_quad, const double *uL, const double4 &r, const double4 &a,
+                                             const double4 &b, double eh_own, double ehR, double side, double nx,
+                                             double ny, const double *t, double *f) {
+    double uR[4], uUp[4], uDn[4];
+    if (nbk >= 0) {
+        uUp[0] = a.x; uUp[1] = a.y; uUp[2] = a.z; uUp[3] = a.w;
+        uDn[0] = b.x; uDn[1] = b.y; uDn[2] = b.z; uDn[3] = b.w;
+        uR[0] = r.x; uR[1] = r.y; uR[2] = r.z; uR[3] = r.w;
+    } else {
+        bc_ghost<double>(P, m, -nbk - 1, g, k, uL, nx, ny, *t, uR);
+        for (int v = 0; v < 4; ++v) { uDn[v] = uL[v]; uUp[v] = uR[v]; }
+        ehR = eh_own;
+    }
+    if (__builtin_expect(!face_flux_exact<FLUX>(K, uL, uDn, uR, uUp, eh_own, ehR, nx, ny, side, f), 0)) {
+        const double4 *pin2 = pin, *nodeP2 = nodeP;
+        asm volatile("" : "+l"(pin2), "+l"(nodeP2));
+        face_flux_plain<FLUX, QUAD>(m, P, pin2, nodeP2, g, k, nbk, dnk, upk, dn2k, up2k, is_quad, t, f);
+    }
+}
+
+// Up and down node values of a face (quads: of its two nodes each, averaged).
+template <bool QUAD>
+__device__ __forceinline__ void face_nodes(const double4 *__restrict__ nodeP, int dnk, int upk, int dn2k, int up2k,
+                                           bool is_quad, double4 &a, double4 &b) {
+    a = nodeP[upk];
+    b = nodeP[dnk];
+    if (QUAD && is_quad) {
+        const double4 a2 = nodeP[up2k], b2 = nodeP[dn2k];
+        a = make_double4(0.5 * (a.x + a2.x), 0.5 * (a.y + a2.y), 0.5 * (a.z + a2.z), 0.5 * (a.w + a2.w));
+        b = make_double4(0.5 * (b.x + b2.x), 0.5 * (b.y + b2.y), 0.5 * (b.z + b2.z), 0.5 * (b.w + b2.w));
+    }
 }
 
 // Face k of cell g, fetching its operands from the per-cell arrays.
@@ -343,34 +439,120 @@ template <int FLUX, bool QUAD>
 __device__ __forceinline__ void face_flux(const DevMesh &m, const DevCase &P, const double4 *__restrict__ pin,
                                           const double4 *__restrict__ nodeP, int64_t g, int k, int nbk,
                                           int dnk, int upk, int dn2k, int up2k, bool is_quad, const double *uL,
-                                          double hx_own, double t, double g2, double *f) {
+                                          double eh_own, const double *t, double *f) {
     const int64_t o = (int64_t)k * m.Nc + g;
     const double side = m.len[o], nx = m.nx[o], ny = m.ny[o];
-    double4 r = make_double4(0.0, 0.0, 0.0, 0.0);
-    double hxR = hx_own;
+    double4 r = make_double4(0.0, 0.0, 0.0, 0.0), a = r, b = r;
+    double ehR = eh_own;
     if (nbk >= 0) {
+        face_nodes<QUAD>(nodeP, dnk, upk, dn2k, up2k, is_quad, a, b);
         r = pin[nbk];
-        if (P.limiter == LIM_VENKAT) hxR = m.hx[nbk];
+        if (P.limiter == LIM_VENKAT) ehR = venkat_half(P.face, m.hx[nbk]);
     }
-    face_flux_at<FLUX, QUAD>(m, P, nodeP, g, k, nbk, dnk, upk, dn2k, up2k, is_quad, uL, r, hx_own, hxR, side, nx, ny,
-                             t, g2, f);
+    face_flux_at<FLUX, QUAD>(m, P, P.face, pin, nodeP, g, k, nbk, dnk, upk, dn2k, up2k, is_quad, uL, r, a, b, eh_own,
+                             ehR, side, nx, ny, t, f);
+}
+
+// The fluxes of a cell's faces summed in face order
+// (calcOneStageMUSCLcpuFast.jl:66-85).  A rolled loop: one face's quotients
+// already overlap, and unrolled the face's code would not stay in the
+// instruction cache.
+template <int FLUX, bool QUAD>
+__device__ __forceinline__ void cell_fluxes(const DevMesh &m, const DevCase &P, const double4 *__restrict__ pin,
+                                            const double4 *__restrict__ nodeP, int64_t g, const int4 &nb, bool is_quad,
+                                            const double *uL, double eh_own, const double *t, double *F) {
+    const int4 dn = m.dn[g], up = m.up[g];
+    int4 dn2 = make_int4(0, 0, 0, 0), up2 = make_int4(0, 0, 0, 0);
+    if (QUAD && is_quad) { dn2 = m.dn2[g]; up2 = m.up2[g]; }
+    const int nf = (QUAD && is_quad) ? 4 : 3;
+#pragma unroll 1
+    for (int k = 0; k < nf; ++k) {
+        double f[4];
+        face_flux<FLUX, QUAD>(m, P, pin, nodeP, g, k, nbr_k(nb, k), nbr_k(dn, k), nbr_k(up, k), nbr_k(dn2, k),
+                              nbr_k(up2, k), is_quad, uL, eh_own, t, f);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) F[v] = k == 0 ? f[v] : F[v] + f[v];
+    }
+}
+
+// A cell's nodes in edge order, where the mesh has them.
+__device__ __forceinline__ int4 cell_nodes(const DevMesh &m, int64_t g) {
+    return m.cn ? ld_once(m.cn + g) : make_int4(0, 0, 0, 0);
+}
+
+// Artificial viscosity of a cell of density rho and size HX whose velocity
+// divergence is divU (calcArtViscosity.jl:46-75); a: the sensor's threshold.
+__device__ __forceinline__ double art_viscosity(double rho, double HX, double divU, double a) {
+    if (-divU > a) {
+        const double tmp = divU * divU - a * a;
+        if (tmp > 0.0) return 0.5 * rho * HX / sqrt(2.0) * HX / sqrt(2.0) * sqrt(tmp) * 1.0e-5;
+    }
+    return 0.0;
+}
+
+// The transport model of diff_source with straight-line quotients
+// (face_exact.cuh); false, and nothing written, where an operand is out of
+// their range or the model is the reference's (whose air conductivity takes
+// a power).
+__device__ __forceinline__ bool diff_model_exact(const DevCase &P, const double4 &me, const double *sx,
+                                                 const double *sy, double du, double dv, double area, double rarea,
+                                                 bool art, double HX, double *diff) {
+    if (P.visc_model == VISC_REFERENCE || !P.face.exact_rows) return false;
+    Numerators n(sx[0]);
+    n.add(sy[0]);
+    double lap[3];
+#pragma unroll
+    for (int v = 0; v < 3; ++v) {
+        lap[v] = div_by(sx[v], area, rarea) + div_by(sy[v], area, rarea);
+        if (v > 0) {
+            n.add(sx[v]);
+            n.add(sy[v]);
+        }
+    }
+    InRange<-150, 200> r(me.w);
+    Divisors<-150, 200> d(me.x);
+    const double yrho = rcp_rn(me.x);
+    double mu = P.mu_ref;
+    if (P.visc_model == VISC_SUTHERLAND) {
+        const double T = div_by(div_by(me.w, me.x, yrho), P.R, P.rR);
+        const double w = 1.0 + div_rn(116.0, T);
+        d.add(T);
+        d.add(w);
+        mu = P.mu_ref * div_by(div_rn(1.4792e-6 * sqrt_rn(T), w), P.suth_ref, P.rsuth);
+    }
+    double divU = 0.0, a = 0.0;
+    if (art) {
+        // (a divergence too small to be rounded right is far above -a)
+        divU = div_by(du, area, rarea) + div_by(dv, area, rarea);
+        const double aS2 = div_by(P.gamma * me.w, me.x, yrho);
+        r.add(aS2);
+        const double root2 = sqrt(2.0);
+        a = div_by(div_rn(0.05 * sqrt_rn(aS2), HX), root2, 1.0 / root2);
+    }
+    if (!n.ok() || !r.ok() || !d.ok()) return false;
+    const double mue = mu + (art ? art_viscosity(me.x, HX, divU, a) : 0.0);
+    diff[1] = mue * lap[0];
+    diff[2] = mue * lap[1];
+    diff[3] = mue * lap[2];
+    return true;
 }
 
 // Second Green-Gauss pass and transport model: the diffusion source of
 // calcDiffTerm (calcDiffTerm.jl:88-113; gradients per calcGradients.jl:36-139,
-// artificial viscosity per calcArtViscosity.jl:46-75).
-template <bool QUAD>
+// artificial viscosity per calcArtViscosity.jl:46-75).  cn: the cell's nodes
+// in edge order (DevMesh::cn), loaded by the caller ahead of its use.
+template <bool QUAD, class Geo>
 __device__ __forceinline__ void diff_source(const DevMesh &m, const DevState &s, const DevCase &P, int64_t g,
-                                            bool is_quad, const double4 &me, double *diff) {
+                                            bool is_quad, const double4 &me, const int4 &cn, const Geo &geo,
+                                            double area, double rarea, double HX, double *diff) {
     const int nf = (QUAD && is_quad) ? 4 : 3;
     double sx[3] = {0.0, 0.0, 0.0}, sy[3] = {0.0, 0.0, 0.0};
     double du = 0.0, dv = 0.0;
     const bool art = (P.visc_model != VISC_REFERENCE) && P.art_visc;
-    for (int k = 0; k < nf; ++k) {
-        const int64_t o = (int64_t)k * m.Nc + g;
-        const double side = m.len[o], nx = m.nx[o], ny = m.ny[o];
-        const int2 e = ld_once(m.c2n + o);
-        const NodeGrad A = s.nodeG[e.x], B = s.nodeG[e.y];
+    // one edge's terms from its two nodes' gradients and velocities
+    auto edge = [&](int k, const NodeGrad &A, const NodeGrad &B, const double2 &na, const double2 &nb) {
+        double nx, ny, side;
+        geo(k, nx, ny, side);
         double fx, fy;
         fx = 0.5 * (A.ru.x + B.ru.x) * -ny * side; fy = 0.5 * (A.ru.y + B.ru.y) * -nx * side;
         sx[0] = (k == 0) ? fx : sx[0] + fx; sy[0] = (k == 0) ? fy : sy[0] + fy;
@@ -379,19 +561,42 @@ __device__ __forceinline__ void diff_source(const DevMesh &m, const DevState &s,
         fx = 0.5 * (A.re.x + B.re.x) * -ny * side; fy = 0.5 * (A.re.y + B.re.y) * -nx * side;
         sx[2] = (k == 0) ? fx : sx[2] + fx; sy[2] = (k == 0) ? fy : sy[2] + fy;
         if (art) {
-            const double4 na = s.nodeP[e.x], nb = s.nodeP[e.y];
-            double fu = 0.5 * (na.y + nb.y) * -nx * side;
-            double fv = 0.5 * (na.z + nb.z) * -ny * side;
+            const double fu = 0.5 * (na.x + nb.x) * -nx * side;
+            const double fv = 0.5 * (na.y + nb.y) * -ny * side;
             du = (k == 0) ? fu : du + fu;
             dv = (k == 0) ? fv : dv + fv;
         }
+    };
+    auto velocity = [&](int n) {
+        return art ? make_double2(s.nodeP[n].y, s.nodeP[n].z) : make_double2(0.0, 0.0);
+    };
+    if (m.cn) {
+        // every node once: a cell's edges are a closed walk over its nodes
+        const NodeGrad A = s.nodeG[cn.x], B = s.nodeG[cn.y], C = s.nodeG[cn.z];
+        const double2 na = velocity(cn.x), nb = velocity(cn.y), nc = velocity(cn.z);
+        edge(0, A, B, na, nb);
+        edge(1, B, C, nb, nc);
+        if (nf == 3) {
+            edge(2, C, A, nc, na);
+        } else {
+            const NodeGrad D = s.nodeG[cn.w];
+            const double2 nd = velocity(cn.w);
+            edge(2, C, D, nc, nd);
+            edge(3, D, A, nd, na);
+        }
+    } else {
+#pragma unroll 1
+        for (int k = 0; k < nf; ++k) {
+            const int2 e = ld_once(m.c2n + (int64_t)k * m.Nc + g);
+            edge(k, s.nodeG[e.x], s.nodeG[e.y], velocity(e.x), velocity(e.y));
+        }
     }
-    const double area = ld_once(m.area + g);
+    diff[0] = 0.0;
+    if (__builtin_expect(diff_model_exact(P, me, sx, sy, du, dv, area, rarea, art, HX, diff), 1)) return;
     double lap[3];
 #pragma unroll
     for (int v = 0; v < 3; ++v) lap[v] = sx[v] / area + sy[v] / area;
     const double T = me.w / me.x / P.R;
-    diff[0] = 0.0;
     if (P.visc_model == VISC_REFERENCE) {
         const double mu = P.mu_ref;
         diff[1] = mu * lap[0];
@@ -401,14 +606,9 @@ __device__ __forceinline__ void diff_source(const DevMesh &m, const DevState &s,
         const double mu = (P.visc_model == VISC_SUTHERLAND) ? P.mu_ref * (sutherland(T) / P.suth_ref) : P.mu_ref;
         double mart = 0.0;
         if (art) {
-            const double HX = ld_once(m.hx + g);
             const double divU = du / area + dv / area;
             const double aS = sqrt(P.gamma * me.w / me.x);
-            const double a = 0.05 * aS / HX / sqrt(2.0);
-            if (-divU > a) {
-                const double tmp = divU * divU - a * a;
-                if (tmp > 0.0) mart = 0.5 * me.x * HX / sqrt(2.0) * HX / sqrt(2.0) * sqrt(tmp) * 1.0e-5;
-            }
+            mart = art_viscosity(me.x, HX, divU, 0.05 * aS / HX / sqrt(2.0));
         }
         // laplacians of u, v and phi = |u|^2/2 + (gamma/Pr) e
         const double mue = mu + (P.art_visc ? mart : 0.0);
@@ -416,6 +616,20 @@ __device__ __forceinline__ void diff_source(const DevMesh &m, const DevState &s,
         diff[2] = mue * lap[1];
         diff[3] = mue * lap[2];
     }
+}
+
+// The same for cell g with everything read from the per-cell arrays.
+template <bool QUAD>
+__device__ __forceinline__ void diff_source_at(const DevMesh &m, const DevState &s, const DevCase &P, int64_t g,
+                                               bool is_quad, const double4 &me, double *diff) {
+    auto geo = [&](int k, double &nx, double &ny, double &side) {
+        const int64_t o = (int64_t)k * m.Nc + g;
+        side = m.len[o];
+        nx = m.nx[o];
+        ny = m.ny[o];
+    };
+    diff_source<QUAD>(m, s, P, g, is_quad, me, cell_nodes(m, g), geo, ld_once(m.area + g), ld_once(m.rarea + g),
+                      ld_once(m.hx + g), diff);
 }
 
 // Euler update (calcOneStageMUSCLcpuFast.jl:94-99), the densityConstrained
@@ -452,11 +666,16 @@ __device__ __forceinline__ void cell_update(const DevMesh &m, const DevState &s,
     st_once(s.U + g, make_double4(Un[0], Un[1], Un[2], Un[3]));
     const double gam = P.gamma;
     const double rho = Un[0];
-    const double ux = Un[1] / Un[0];
-    const double uy = Un[2] / Un[0];
-    const double p = (gam - 1.0) * (Un[3] - 0.5 * (Un[1] * Un[1] + Un[2] * Un[2]) / Un[0]);
-    const double a = sqrt(gam * p / rho);
-    const double vmax = sqrt(ux * ux + uy * uy) + a;
+    CellPrims q;
+    if (__builtin_expect(!(prims_exact(Un, gam, in.charlen, q) && P.face.exact_rows), 0)) {
+        q.ux = Un[1] / Un[0];
+        q.uy = Un[2] / Un[0];
+        q.p = (gam - 1.0) * (Un[3] - 0.5 * (Un[1] * Un[1] + Un[2] * Un[2]) / Un[0]);
+        const double a = sqrt(gam * q.p / rho);
+        q.vmax = sqrt(q.ux * q.ux + q.uy * q.uy) + a;
+        q.rmin = in.charlen / q.vmax;
+    }
+    const double ux = q.ux, uy = q.uy, p = q.p;
     pout[g] = make_double4(rho, ux, uy, p);
     const double area = in.area;
 #pragma unroll
@@ -466,8 +685,8 @@ __device__ __forceinline__ void cell_update(const DevMesh &m, const DevState &s,
         part.tot[v] = Un[v] * area;
     }
     part.ek = 0.5 * rho * (ux * ux + uy * uy) * area;
-    part.vmax = vmax;
-    part.rmin = in.charlen / vmax;
+    part.vmax = q.vmax;
+    part.rmin = q.rmin;
     part.rhomin = me.x;
     part.rhomax = me.x;
     const bool ok = isfinite(Un[0]) && isfinite(Un[1]) && isfinite(Un[2]) && isfinite(Un[3]) && (rho > 0.0) &&
@@ -479,7 +698,7 @@ __device__ __forceinline__ void cell_update(const DevMesh &m, const DevState &s,
 
 template <int FLUX, bool VISC, bool QUAD, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_cell_step(const DevMesh m, const DevState s) {
-    __shared__ double s_red[kPartFields * 256];
+    __shared__ double s_red[8 * kPartials];
     const int par = *s.parity;
     const double4 *__restrict__ pin = s.prim + (int64_t)par * m.Nc;
     double4 *__restrict__ pout = s.prim + (int64_t)(par ^ 1) * m.Nc;
@@ -487,7 +706,7 @@ __global__ void __launch_bounds__(256, MINB) k_cell_step(const DevMesh m, const 
     for (int64_t tile = blockIdx.x; tile < m.ntiles; tile += gridDim.x) {
         const int c = m.tile_case[tile];
         const DevCase &P = m.cases[c];
-        const double dt = s.cstate[c].dt, t = s.cstate[c].t;
+        const double dt = s.cstate[c].dt;
         const int64_t g = tile * blockDim.x + threadIdx.x;
         Part part;
         part.init();
@@ -496,27 +715,11 @@ __global__ void __launch_bounds__(256, MINB) k_cell_step(const DevMesh m, const 
             const bool is_quad = QUAD && (nb.w != kAbsent);
             const double4 me = pin[g];
             const double uL[4] = {me.x, me.y, me.z, me.w};
-            const double gam = P.gamma;
-            const double g2 = 2.0 * (gam - 1.0) / (gam + 1.0);
-            const double hx_own = (P.limiter == LIM_VENKAT) ? m.hx[g] : 0.0;
-            const int4 dn = m.dn[g], up = m.up[g];
-            int4 dn2 = make_int4(0, 0, 0, 0), up2 = make_int4(0, 0, 0, 0);
-            if (QUAD && is_quad) { dn2 = m.dn2[g]; up2 = m.up2[g]; }
-            double F[4], f[4];
-            face_flux<FLUX, QUAD>(m, P, pin, nodeP, g, 0, nb.x, dn.x, up.x, dn2.x, up2.x, is_quad, uL, hx_own, t, g2, F);
-            face_flux<FLUX, QUAD>(m, P, pin, nodeP, g, 1, nb.y, dn.y, up.y, dn2.y, up2.y, is_quad, uL, hx_own, t, g2, f);
-#pragma unroll
-            for (int v = 0; v < 4; ++v) F[v] = F[v] + f[v];
-            face_flux<FLUX, QUAD>(m, P, pin, nodeP, g, 2, nb.z, dn.z, up.z, dn2.z, up2.z, is_quad, uL, hx_own, t, g2, f);
-#pragma unroll
-            for (int v = 0; v < 4; ++v) F[v] = F[v] + f[v];
-            if (QUAD && is_quad) {
-                face_flux<FLUX, QUAD>(m, P, pin, nodeP, g, 3, nb.w, dn.w, up.w, dn2.w, up2.w, is_quad, uL, hx_own, t, g2, f);
-#pragma unroll
-                for (int v = 0; v < 4; ++v) F[v] = F[v] + f[v];
-            }
+            const double eh_own = (P.limiter == LIM_VENKAT) ? venkat_half(P.face, m.hx[g]) : 0.0;
+            double F[4];
+            cell_fluxes<FLUX, QUAD>(m, P, pin, nodeP, g, nb, is_quad, uL, eh_own, &s.cstate[c].t, F);
             double diff[4] = {0.0, 0.0, 0.0, 0.0};
-            if (VISC) diff_source<QUAD>(m, s, P, g, is_quad, me, diff);
+            if (VISC) diff_source_at<QUAD>(m, s, P, g, is_quad, me, diff);
             cell_update(m, s, P, g, me, F, diff, dt, load_cell_in(m, s, g), pout, part);
         }
         tile_record<true, false>(m, s, tile, part, s_red);
@@ -524,90 +727,90 @@ __global__ void __launch_bounds__(256, MINB) k_cell_step(const DevMesh m, const 
 }
 
 // The fused cell kernel over tile-local face lists (GD2D_LOOP_TILE_FACES).
-// Phase 1 stages the tile's primitives (and HX) in shared memory; phase 2
-// runs the tile's face list, one face per thread: a face between two cells
-// of the tile is computed once, from its lower-indexed cell, and its flux
-// stored negated into the other cell's slot -- exact because the listed
-// pairs are only those whose face state and flux are antisymmetric bit for
-// bit under exchange of the two cells (checked on the host: AUSM+ with the
-// Minmod or Venkatakrishnan limiter or none, negated normals, exchanged
-// down/up nodes); every other face slot is computed from its own cell as in
-// k_cell_step.  Phase 3 sums each cell's slots in face order
-// (calcOneStageMUSCLcpuFast.jl:66-85) and finishes the cell as k_cell_step.
+// Phase 1 stages the tile's primitives (and the limiter's scale) in shared
+// memory; phase 2 runs the tile's face list, one face per thread: a face
+// between two cells of the tile is computed once, from its lower-indexed
+// cell, and its flux stored negated into the other cell's slot -- exact
+// because the listed pairs are only those whose face state and flux are
+// antisymmetric bit for bit under exchange of the two cells (checked on the
+// host: AUSM+ with the Minmod or Venkatakrishnan limiter or none, negated
+// normals, exchanged down/up nodes); every other face slot is computed from
+// its own cell as in k_cell_step.  Phase 3 sums each cell's slots in face
+// order (calcOneStageMUSCLcpuFast.jl:66-85) and finishes the cell as
+// k_cell_step.
+//
+// What bounds it (2.09M-cell viscous cylinder, 276 us; 365 before the
+// divisions went into straight-line rows): issue and latency together.  Half
+// the issue slots and 40% of the FP64 pipe are used; with all arithmetic
+// taken out 184 us remain, with the face loop taken out 191, so a tile's
+// gathers and its arithmetic overlap only across the three blocks of an SM.
 template <int FLUX, bool VISC, bool QUAD, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_cell_step_tf(const DevMesh m, const DevState s) {
     constexpr int NS = QUAD ? 4 : 3;
-    // one buffer: the tile's primitives, then its flux slots; the step
-    // reduction reuses it once both have been consumed
+    // the tile's primitives, then its flux slots, which the step reduction
+    // reuses once they have been consumed
     __shared__ double4 s_mem[(1 + NS) * 256];
-    __shared__ double s_hx[256];
-    static_assert((1 + NS) * 256 * 4 >= kPartFields * 256, "reduction buffer");
+    __shared__ double s_eh[256];  // venkat_half of the tile's cells
+    __shared__ FaceCase s_face;
     double4 *const s_prim = s_mem;
     double4 (*const s_flux)[256] = reinterpret_cast<double4 (*)[256]>(s_mem + 256);
+    const int B = blockDim.x, tid = threadIdx.x;
     pdl_trigger();
-    pdl_wait();
-    const int par = *s.parity;
-    const double4 *__restrict__ pin = s.prim + (int64_t)par * m.Nc;
-    double4 *__restrict__ pout = s.prim + (int64_t)(par ^ 1) * m.Nc;
-    const int B = blockDim.x;
     for (int64_t tile = blockIdx.x; tile < m.ntiles; tile += gridDim.x) {
         const int64_t base = tile * B;
-        const int64_t g = base + threadIdx.x;
-        // loads that depend on nothing go out first: the face-list bounds
-        // and HX (used only with the Venkatakrishnan limiter) need not wait
-        // for the case record
-        const int64_t f0 = m.tf_off[tile], f1 = m.tf_off[tile + 1];
-        s_prim[threadIdx.x] = pin[g];
-        s_hx[threadIdx.x] = ld_once(m.hx + g);
+        const int64_t g = base + tid;
+        // the mesh does not depend on the kernel before this one: what a
+        // tile reads of it first is asked for before the wait
+        const int fb = (int)m.tf_off[tile] + tid, fe = (int)m.tf_off[tile + 1];
+        int4 next = make_int4(0, 0, 0, 0), cn = next;
+        if (fb < fe) next = ld_once(m.tf_rec + fb);
+        if (VISC) cn = cell_nodes(m, g);
+        const double eh = m.eh[g];
         const int c = m.tile_case[tile];
         const DevCase &P = m.cases[c];
-        const double t = s.cstate[c].t;
-        const bool venkat = P.limiter == LIM_VENKAT;
-        // face indices fit 32 bits (setup checks the total); the first face
-        // record goes out with the staging loads and each next one before
-        // the current face's gathers, so no face waits for its record
-        const int fb = (int)f0 + (int)threadIdx.x, fe = (int)f1;
-        int4 next = make_int4(0, 0, 0, 0);
-        if (fb < fe) next = ld_once(m.tf_rec + fb);
+        double faceconst = 0.0;
+        if (tid < (int)(sizeof(FaceCase) / 8)) faceconst = reinterpret_cast<const double *>(&P.face)[tid];
+        if (tile == blockIdx.x) pdl_wait();
+        const int par = *s.parity;
+        const double4 *__restrict__ pin = s.prim + (int64_t)par * m.Nc;
+        double4 *__restrict__ pout = s.prim + (int64_t)(par ^ 1) * m.Nc;
+        s_prim[tid] = pin[g];
+        s_eh[tid] = eh;
+        if (tid < (int)(sizeof(FaceCase) / 8)) reinterpret_cast<double *>(&s_face)[tid] = faceconst;
         __syncthreads();
-        const double gam = P.gamma;
-        const double g2 = 2.0 * (gam - 1.0) / (gam + 1.0);
         for (int f = fb; f < fe; f += B) {
             const int4 rec = next;
             if (f + B < fe) next = ld_once(m.tf_rec + f + B);
             const TileFace tf = unpack_tile_face(rec.y);
             const double4 a4 = s_prim[tf.la];
             const double uL[4] = {a4.x, a4.y, a4.z, a4.w};
-            const double hx_own = venkat ? s_hx[tf.la] : 0.0;
-            double4 r = make_double4(0.0, 0.0, 0.0, 0.0);
-            double hxR = hx_own;
+            const double eh_own = s_eh[tf.la];
+            double4 r = make_double4(0.0, 0.0, 0.0, 0.0), up = r, down = r;
+            double ehR = eh_own;
+            int2 q2 = make_int2(0, 0);
+            if (QUAD && tf.quad) q2 = m.tf_q[f];
             if (rec.x >= 0) {
+                face_nodes<QUAD>(s.nodeP, rec.z, rec.w, q2.x, q2.y, QUAD && tf.quad, up, down);
                 const int64_t lr = (int64_t)rec.x - base;
                 if (lr >= 0 && lr < B) {
                     r = s_prim[lr];
-                    if (venkat) hxR = s_hx[lr];
+                    ehR = s_eh[lr];
                 } else {
                     r = pin[rec.x];
-                    if (venkat) hxR = m.hx[rec.x];
+                    ehR = m.eh[rec.x];
                 }
             }
-            int2 q2 = make_int2(0, 0);
-            if (QUAD && tf.quad) q2 = m.tf_q[f];
-            double fv[4];
-            // the face geometry of slot (la, ka) from the per-cell planes,
-            // cached: the viscous source reads the same lines again
             const int64_t og = (int64_t)tf.ka * m.Nc + base + tf.la;
-            face_flux_at<FLUX, QUAD>(m, P, s.nodeP, base + tf.la, tf.ka, rec.x, rec.z, rec.w, q2.x, q2.y,
-                                     QUAD && tf.quad, uL, r, hx_own, hxR, m.len[og], m.nx[og], m.ny[og], t,
-                                     g2, fv);
+            double fv[4];
+            face_flux_at<FLUX, QUAD>(m, P, s_face, pin, s.nodeP, base + tf.la, tf.ka, rec.x, rec.z, rec.w, q2.x, q2.y,
+                                     QUAD && tf.quad, uL, r, up, down, eh_own, ehR, m.len[og], m.nx[og], m.ny[og],
+                                     &s.cstate[c].t, fv);
             s_flux[tf.ka][tf.la] = make_double4(fv[0], fv[1], fv[2], fv[3]);
             if (tf.lbp) s_flux[tf.kb][tf.lbp - 1] = make_double4(-fv[0], -fv[1], -fv[2], -fv[3]);
         }
         // the cell's viscous source needs no flux: evaluated before the
         // barrier, it fills the time a thread with fewer faces would wait
-        // (the cell's primitives are re-read from the stage rather than
-        // held in registers through the face phase)
-        const double4 me = s_prim[threadIdx.x];
+        const double4 me = s_prim[tid];
         const double dt = s.cstate[c].dt;
         // triangles: the viscous source is evaluated for padding cells too
         // (node 0 in their edge slots, zero area; the result is unused), and
@@ -620,7 +823,15 @@ __global__ void __launch_bounds__(256, MINB) k_cell_step_tf(const DevMesh m, con
             is_quad = nb.w != kAbsent;
         }
         double diff[4] = {0.0, 0.0, 0.0, 0.0};
-        if (VISC && live) diff_source<QUAD>(m, s, P, g, is_quad, me, diff);
+        if (VISC && live) {
+            auto geo = [&](int k, double &nx, double &ny, double &side) {
+                const int64_t o = (int64_t)k * m.Nc + g;
+                side = m.len[o];
+                nx = m.nx[o];
+                ny = m.ny[o];
+            };
+            diff_source<QUAD>(m, s, P, g, is_quad, me, cn, geo, m.area[g], m.rarea[g], ld_once(m.hx + g), diff);
+        }
         // the update's own loads go out before the barrier (padded arrays:
         // in bounds for padding cells, whose values are not used)
         const CellIn cin = load_cell_in(m, s, g);
@@ -629,16 +840,18 @@ __global__ void __launch_bounds__(256, MINB) k_cell_step_tf(const DevMesh m, con
         Part part;
         part.init();
         if (live) {
-            const double4 a0 = s_flux[0][threadIdx.x], a1 = s_flux[1][threadIdx.x], a2 = s_flux[2][threadIdx.x];
+            const double4 a0 = s_flux[0][tid], a1 = s_flux[1][tid], a2 = s_flux[2][tid];
             double F[4] = {a0.x + a1.x, a0.y + a1.y, a0.z + a1.z, a0.w + a1.w};
             F[0] = F[0] + a2.x; F[1] = F[1] + a2.y; F[2] = F[2] + a2.z; F[3] = F[3] + a2.w;
             if (QUAD && is_quad) {
-                const double4 a3 = s_flux[NS - 1][threadIdx.x];
+                const double4 a3 = s_flux[NS - 1][tid];
                 F[0] = F[0] + a3.x; F[1] = F[1] + a3.y; F[2] = F[2] + a3.z; F[3] = F[3] + a3.w;
             }
             cell_update(m, s, P, g, me, F, diff, dt, cin, pout, part);
         }
-        tile_record<true, true>(m, s, tile, part, reinterpret_cast<double *>(s_mem));
+        // (every thread has read the primitives: the reduction's shares go
+        // there, clear of the flux slots still being read)
+        tile_record<true, false>(m, s, tile, part, reinterpret_cast<double *>(s_prim));
     }
 }
 
@@ -739,6 +952,7 @@ template <bool QUAD>
 __global__ void __launch_bounds__(256, GD2D_NODE_MINB) k_grad1_cells(const DevMesh m, const DevState s) {
     constexpr int NF = QUAD ? 4 : 3;
     pdl_trigger();
+    const bool exact = m.exact_rows != 0;
     pdl_wait();
     for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < m.Nc; g += (int64_t)gridDim.x * blockDim.x) {
         // Every per-cell load is issued before any of them is tested, so a
@@ -748,20 +962,18 @@ __global__ void __launch_bounds__(256, GD2D_NODE_MINB) k_grad1_cells(const DevMe
         const double area = ld_once(m.area + g);
         double side[NF], nx[NF], ny[NF];
         int2 e[NF];
+        const int4 cn = cell_nodes(m, g);
 #pragma unroll
         for (int k = 0; k < NF; ++k) {
             const int64_t o = (int64_t)k * m.Nc + g;
             side[k] = ld_once(m.len + o);
             nx[k] = ld_once(m.nx + o);
             ny[k] = ld_once(m.ny + o);
-            e[k] = ld_once(m.c2n + o);
+            if (!m.cn) e[k] = ld_once(m.c2n + o);
         }
         const int nf = (QUAD && side[NF - 1] != 0.0) ? 4 : 3;
         double sx[3] = {0.0, 0.0, 0.0}, sy[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-        for (int k = 0; k < NF; ++k) {
-            if (k >= nf) break;
-            const double4 A = s.nodeC[e[k].x], B = s.nodeC[e[k].y];
+        auto edge = [&](int k, const double4 &A, const double4 &B) {
             double fx, fy;
             fx = 0.5 * (A.x + B.x) * -ny[k] * side[k]; fy = 0.5 * (A.x + B.x) * -nx[k] * side[k];
             sx[0] = (k == 0) ? fx : sx[0] + fx; sy[0] = (k == 0) ? fy : sy[0] + fy;
@@ -769,12 +981,47 @@ __global__ void __launch_bounds__(256, GD2D_NODE_MINB) k_grad1_cells(const DevMe
             sx[1] = (k == 0) ? fx : sx[1] + fx; sy[1] = (k == 0) ? fy : sy[1] + fy;
             fx = 0.5 * (A.z + B.z) * -ny[k] * side[k]; fy = 0.5 * (A.z + B.z) * -nx[k] * side[k];
             sx[2] = (k == 0) ? fx : sx[2] + fx; sy[2] = (k == 0) ? fy : sy[2] + fy;
+        };
+        if (m.cn) {
+            const double4 A = s.nodeC[cn.x], B = s.nodeC[cn.y], C = s.nodeC[cn.z];
+            edge(0, A, B);
+            edge(1, B, C);
+            if (nf == 3) {
+                edge(2, C, A);
+            } else {
+                const double4 D = s.nodeC[cn.w];
+                edge(2, C, D);
+                edge(NF - 1, D, A);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < NF; ++k)
+                if (k < nf) edge(k, s.nodeC[e[k].x], s.nodeC[e[k].y]);
         }
         if (area == 0.0) continue;
+        // six quotients over one area (face_exact.cuh's range: the area's is
+        // the case's, a sum too small to be divided right takes the plain `/`)
+        const double y = rcp_rn(area);
+        double qx[3], qy[3];
+        Numerators n(sx[0]);
+        n.add(sy[0]);
+#pragma unroll
+        for (int v = 0; v < 3; ++v) {
+            qx[v] = div_by(sx[v], area, y);
+            qy[v] = div_by(sy[v], area, y);
+            if (v > 0) {
+                n.add(sx[v]);
+                n.add(sy[v]);
+            }
+        }
+        if (__builtin_expect(!(exact && n.ok()), 0)) {
+#pragma unroll
+            for (int v = 0; v < 3; ++v) { qx[v] = sx[v] / area; qy[v] = sy[v] / area; }
+        }
         NodeGrad r;
-        r.ru = make_double2(sx[0] / area, sy[0] / area);
-        r.rv = make_double2(sx[1] / area, sy[1] / area);
-        r.re = make_double2(sx[2] / area, sy[2] / area);
+        r.ru = make_double2(qx[0], qy[0]);
+        r.rv = make_double2(qx[1], qy[1]);
+        r.re = make_double2(qx[2], qy[2]);
         s.g1[g] = r;
     }
 }
@@ -821,7 +1068,7 @@ static __global__ void __launch_bounds__(256, GD2D_NODE_MINB) k_grad1_nodes(cons
 // phs2dcns2dcellsSA (utilsFVM2dp.jl:4-17) on the current primitives and the
 // reductions that give the first step's dt (createFields2d's VMAX).
 static __global__ void __launch_bounds__(256) k_init_state(const DevMesh m, const DevState s, int64_t t0, int64_t t1) {
-    __shared__ double s_red[kPartFields * 256];
+    __shared__ double s_red[8 * kPartials];
     const int par = *s.parity;
     const double4 *__restrict__ pin = s.prim + (int64_t)par * m.Nc;
     for (int64_t tile = t0 + blockIdx.x; tile < t1; tile += gridDim.x) {
@@ -864,20 +1111,17 @@ __global__ void __launch_bounds__(256) k_face_flux(const DevMesh m, const DevSta
     const int nbk = fc.y, ka = fc.z & 255, kb = fc.z >> 8;
     const int c = m.tile_case[a / tile_cells];
     const DevCase &P = m.cases[c];
-    const double t = s.cstate[c].t;
     const int4 nb = m.nbr[a];
     const bool is_quad = QUAD && (nb.w != kAbsent);
     const double4 me = pin[a];
     const double uL[4] = {me.x, me.y, me.z, me.w};
-    const double gam = P.gamma;
-    const double g2 = 2.0 * (gam - 1.0) / (gam + 1.0);
-    const double hx_own = (P.limiter == LIM_VENKAT) ? m.hx[a] : 0.0;
+    const double eh_own = (P.limiter == LIM_VENKAT) ? venkat_half(P.face, m.hx[a]) : 0.0;
     const int4 dn = m.dn[a], up = m.up[a];
     int4 dn2 = make_int4(0, 0, 0, 0), up2 = make_int4(0, 0, 0, 0);
     if (QUAD && is_quad) { dn2 = m.dn2[a]; up2 = m.up2[a]; }
     double fv[4];
     face_flux<FLUX, QUAD>(m, P, pin, s.nodeP, a, ka, nbk, nbr_k(dn, ka), nbr_k(up, ka), nbr_k(dn2, ka),
-                          nbr_k(up2, ka), is_quad, uL, hx_own, t, g2, fv);
+                          nbr_k(up2, ka), is_quad, uL, eh_own, &s.cstate[c].t, fv);
     if (SLOTS) {
         Fslot[(int64_t)ka * m.Nc + a] = make_double4(fv[0], fv[1], fv[2], fv[3]);
         if (nbk >= 0) Fslot[(int64_t)kb * m.Nc + nbk] = make_double4(-fv[0], -fv[1], -fv[2], -fv[3]);
@@ -899,7 +1143,7 @@ template <bool VISC, bool QUAD, bool SLOTS, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_face_update(const DevMesh m, const DevState s,
                                                           double4 *__restrict__ Facc,
                                                           const double4 *__restrict__ Fslot) {
-    __shared__ double s_red[kPartFields * 256];
+    __shared__ double s_red[8 * kPartials];
     const int par = *s.parity;
     const double4 *__restrict__ pin = s.prim + (int64_t)par * m.Nc;
     double4 *__restrict__ pout = s.prim + (int64_t)(par ^ 1) * m.Nc;
@@ -929,7 +1173,7 @@ __global__ void __launch_bounds__(256, MINB) k_face_update(const DevMesh m, cons
                 Facc[g] = make_double4(0.0, 0.0, 0.0, 0.0);
             }
             double diff[4] = {0.0, 0.0, 0.0, 0.0};
-            if (VISC) diff_source<QUAD>(m, s, P, g, is_quad, me, diff);
+            if (VISC) diff_source_at<QUAD>(m, s, P, g, is_quad, me, diff);
             cell_update(m, s, P, g, me, F, diff, dt, load_cell_in(m, s, g), pout, part);
         }
         tile_record<true, false>(m, s, tile, part, s_red);
@@ -957,22 +1201,9 @@ __global__ void __launch_bounds__(256) k_stage_only(const DevMesh m, const DevSt
     const bool is_quad = QUAD && (nb.w != kAbsent);
     const double4 me = pin[g];
     const double uL[4] = {me.x, me.y, me.z, me.w};
-    const double gam = P.gamma;
-    const double g2 = 2.0 * (gam - 1.0) / (gam + 1.0);
-    const double hx_own = (P.limiter == LIM_VENKAT) ? m.hx[g] : 0.0;
-    const int4 dn = m.dn[g], up = m.up[g];
-    int4 dn2 = make_int4(0, 0, 0, 0), up2 = make_int4(0, 0, 0, 0);
-    if (QUAD && is_quad) { dn2 = m.dn2[g]; up2 = m.up2[g]; }
-    double F[4], f[4];
-    face_flux<FLUX, QUAD>(m, P, pin, s.nodeP, g, 0, nb.x, dn.x, up.x, dn2.x, up2.x, is_quad, uL, hx_own, t, g2, F);
-    face_flux<FLUX, QUAD>(m, P, pin, s.nodeP, g, 1, nb.y, dn.y, up.y, dn2.y, up2.y, is_quad, uL, hx_own, t, g2, f);
-    for (int v = 0; v < 4; ++v) F[v] = F[v] + f[v];
-    face_flux<FLUX, QUAD>(m, P, pin, s.nodeP, g, 2, nb.z, dn.z, up.z, dn2.z, up2.z, is_quad, uL, hx_own, t, g2, f);
-    for (int v = 0; v < 4; ++v) F[v] = F[v] + f[v];
-    if (QUAD && is_quad) {
-        face_flux<FLUX, QUAD>(m, P, pin, s.nodeP, g, 3, nb.w, dn.w, up.w, dn2.w, up2.w, is_quad, uL, hx_own, t, g2, f);
-        for (int v = 0; v < 4; ++v) F[v] = F[v] + f[v];
-    }
+    const double eh_own = (P.limiter == LIM_VENKAT) ? venkat_half(P.face, m.hx[g]) : 0.0;
+    double F[4];
+    cell_fluxes<FLUX, QUAD>(m, P, pin, s.nodeP, g, nb, is_quad, uL, eh_own, &t, F);
     double diff[4] = {0.0, 0.0, 0.0, 0.0};
     if (diffs) {
         const double4 d = diffs[g];
@@ -1024,7 +1255,7 @@ __global__ void __launch_bounds__(256) k_diff_only(const DevMesh m, const DevSta
     const int4 nb = m.nbr[g];
     if (nb.x == kAbsent) return;
     double diff[4];
-    diff_source<QUAD>(m, s, P, g, QUAD && nb.w != kAbsent, pin[g], diff);
+    diff_source_at<QUAD>(m, s, P, g, QUAD && nb.w != kAbsent, pin[g], diff);
     diffs[g] = make_double4(diff[0], diff[1], diff[2], diff[3]);
 }
 
