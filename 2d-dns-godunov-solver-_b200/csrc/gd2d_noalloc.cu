@@ -15,10 +15,16 @@
 // state (evaluate2d.jl:87-93), Delta = Unew - Uold and Uold <- Unew
 // (:95-104), and the per-variable residual sum of Delta^2 with the largest
 // VMAX (updateResidualSA, evaluate2d.jl:17-20) through a two-level
-// reduction: one record per 256-cell tile in the scratch array, then the
-// block that finishes last (elected by a ticket counter in the same array)
-// reduces the records in a fixed order.  Built with -fmad=false like the
-// other FP64 kernels.
+// reduction: one record per block in the scratch array, then the block that
+// finishes last (elected by a ticket counter in the same array) reduces the
+// records in a fixed order.  Built with -fmad=false like the other FP64
+// kernels.
+//
+// Bound: memory, 128 bytes a cell.  The blocks that fit the device at once
+// each take every gridDim-th stretch of 256 cells and keep their sums in
+// registers, so that there are a few hundred records: with one block, one
+// fence and one record per 256 cells, and one block to fold them, 4.2M cells
+// took 790 us (0.68 TB/s).
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -26,6 +32,7 @@
 #include <mutex>
 
 #include "../../include/godunov2d.h"
+#include "face_exact.cuh"
 #include "gd2d_internal.h"
 
 namespace {
@@ -34,6 +41,7 @@ constexpr int64_t kNoAllocMaxCells = int64_t(1) << 24;  // 16,777,216 cells
 constexpr int kNoAllocTile = 256;
 constexpr int64_t kNoAllocMaxTiles = kNoAllocMaxCells / kNoAllocTile;  // 65,536
 constexpr int kRec = 8;  // res[4], vmax, bad, 2 spare
+constexpr int kNoAllocBlocksPerSm = 4;
 // Records, then 256 bytes holding the ticket counter (first 4 bytes).
 constexpr int64_t kScratchDoubles = kNoAllocMaxTiles * kRec + 32;
 
@@ -79,44 +87,47 @@ __device__ __forceinline__ void red_block(Red &a, Red *sh) {
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(kNoAllocTile)
+__global__ void __launch_bounds__(kNoAllocTile, kNoAllocBlocksPerSm)
 k_update_variables_noalloc(const double *__restrict__ unew, double *__restrict__ uold, double *__restrict__ prims,
-                           int64_t n, double G, double *scratch, int64_t ntiles, double *stats_out) {
+                           int64_t n, double G, double *scratch, double *stats_out) {
     __shared__ Red sh[kNoAllocTile / 32];
     __shared__ int s_last;
     unsigned int *ticket = reinterpret_cast<unsigned int *>(scratch + kNoAllocMaxTiles * kRec);
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     Red a{0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    if (i < n) {
-        const double U1 = unew[i], U2 = unew[n + i], U3 = unew[2 * n + i], U4 = unew[3 * n + i];
-        const double rho = U1;
-        const double ux = U2 / U1;
-        const double uy = U3 / U1;
-        const double p = (G - 1.0) * (U4 - 0.5 * (U2 * U2 + U3 * U3) / U1);
-        const double as = sqrt(G * p / rho);
-        const double vmax = sqrt(ux * ux + uy * uy) + as;
-        prims[i] = rho; prims[n + i] = ux; prims[2 * n + i] = uy; prims[3 * n + i] = p;
-        const double d0 = U1 - uold[i], d1 = U2 - uold[n + i], d2 = U3 - uold[2 * n + i], d3 = U4 - uold[3 * n + i];
-        uold[i] = U1; uold[n + i] = U2; uold[2 * n + i] = U3; uold[3 * n + i] = U4;
-        a.r0 = d0 * d0; a.r1 = d1 * d1; a.r2 = d2 * d2; a.r3 = d3 * d3;
-        a.vmax = vmax;
-        const bool ok = isfinite(U1) && isfinite(U2) && isfinite(U3) && isfinite(U4) && rho > 0.0 && p > 0.0;
-        a.bad = ok ? 0.0 : 1.0;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        const double U[4] = {__ldcs(unew + i), __ldcs(unew + n + i), __ldcs(unew + 2 * n + i), __ldcs(unew + 3 * n + i)};
+        const double O[4] = {__ldcs(uold + i), __ldcs(uold + n + i), __ldcs(uold + 2 * n + i), __ldcs(uold + 3 * n + i)};
+        gd2d::CellPrims q;
+        if (__builtin_expect(!gd2d::prims_exact(U, G, 1.0, q), 0)) {
+            q.ux = U[1] / U[0];
+            q.uy = U[2] / U[0];
+            q.p = (G - 1.0) * (U[3] - 0.5 * (U[1] * U[1] + U[2] * U[2]) / U[0]);
+            q.vmax = sqrt(q.ux * q.ux + q.uy * q.uy) + sqrt(G * q.p / U[0]);
+        }
+        __stcs(prims + i, U[0]); __stcs(prims + n + i, q.ux);
+        __stcs(prims + 2 * n + i, q.uy); __stcs(prims + 3 * n + i, q.p);
+        const double d0 = U[0] - O[0], d1 = U[1] - O[1], d2 = U[2] - O[2], d3 = U[3] - O[3];
+        __stcs(uold + i, U[0]); __stcs(uold + n + i, U[1]);
+        __stcs(uold + 2 * n + i, U[2]); __stcs(uold + 3 * n + i, U[3]);
+        a.r0 += d0 * d0; a.r1 += d1 * d1; a.r2 += d2 * d2; a.r3 += d3 * d3;
+        a.vmax = fmax(a.vmax, q.vmax);
+        const bool ok = isfinite(U[0]) && isfinite(U[1]) && isfinite(U[2]) && isfinite(U[3]) && U[0] > 0.0 && q.p > 0.0;
+        if (!ok) a.bad = 1.0;
     }
     red_block(a, sh);
     if (threadIdx.x == 0) {
         double *rec = scratch + (int64_t)blockIdx.x * kRec;
         rec[0] = a.r0; rec[1] = a.r1; rec[2] = a.r2; rec[3] = a.r3; rec[4] = a.vmax; rec[5] = a.bad;
         __threadfence();
-        const unsigned int prev = atomicAdd(ticket, 1u);
-        s_last = (prev == (unsigned int)(ntiles - 1)) ? 1 : 0;
+        s_last = (atomicAdd(ticket, 1u) == gridDim.x - 1u) ? 1 : 0;
     }
     __syncthreads();
     if (!s_last) return;
     __threadfence();
     Red acc{0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    for (int64_t t = threadIdx.x; t < ntiles; t += blockDim.x) {
-        const double *rec = scratch + t * kRec;
+    for (unsigned int t = threadIdx.x; t < gridDim.x; t += blockDim.x) {
+        const double *rec = scratch + (int64_t)t * kRec;
         Red b{__ldcg(rec), __ldcg(rec + 1), __ldcg(rec + 2), __ldcg(rec + 3), __ldcg(rec + 4), __ldcg(rec + 5)};
         red_combine(acc, b);
     }
@@ -224,8 +235,12 @@ extern "C" int gd2d_update_variables_noalloc(const double *d_unew, double *d_uol
     // the ticket counter must start at zero (a previous call may have failed)
     e = cudaMemsetAsync(scratch + kNoAllocMaxTiles * kRec, 0, 256, st);
     if (e != cudaSuccess) return noalloc_fail(GD2D_ERR_CUDA, cudaGetErrorString(e));
-    k_update_variables_noalloc<<<(unsigned int)ntiles, kNoAllocTile, 0, st>>>(d_unew, d_uold, d_prims, n_cells, gamma,
-                                                                            scratch, ntiles, d_stats);
+    int sms = 0;
+    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return noalloc_fail(GD2D_ERR_CUDA, cudaGetErrorString(e));
+    const int64_t blocks = ntiles < (int64_t)sms * kNoAllocBlocksPerSm ? ntiles : (int64_t)sms * kNoAllocBlocksPerSm;
+    k_update_variables_noalloc<<<(unsigned int)blocks, kNoAllocTile, 0, st>>>(d_unew, d_uold, d_prims, n_cells, gamma,
+                                                                             scratch, d_stats);
     e = cudaGetLastError();
     if (e != cudaSuccess) return noalloc_fail(GD2D_ERR_CUDA, cudaGetErrorString(e));
     return GD2D_OK;
