@@ -769,7 +769,7 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
     // cells of the same kind and exactly one slot of each facing the other
     std::vector<int64_t> tf_off;
     std::vector<int4> tf_rec;
-    std::vector<int2> tf_q, tf_e;
+    std::vector<int2> tf_q;
     std::vector<double> tf_nx, tf_ny, tf_len;
     if (h->loop == GD2D_LOOP_TILE_FACES) {
         std::vector<char> case_pairs(n_cases, 0);
@@ -796,12 +796,6 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
             if (is_quad_cell(lo) && (code_k(dn2[hi], khi) != code_k(up2[lo], klo) ||
                                      code_k(up2[hi], khi) != code_k(dn2[lo], klo)))
                 return false;
-            // the viscous edge terms are negated for the other cell too: the
-            // two slots name the same pair of edge nodes (in either order)
-            if (h->visc) {
-                const int2 el = c2n[ol], eh = c2n[oh];
-                if (!((el.x == eh.x && el.y == eh.y) || (el.x == eh.y && el.y == eh.x))) return false;
-            }
             return true;
         };
         tf_off.assign(ntiles + 1, 0);
@@ -834,7 +828,6 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
                     if (h->quads) tf_q.push_back(make_int2(code_k(dn2[g], k), code_k(up2[g], k)));
                     if (!h->mixed) continue;  // the FP64 kernel reads the per-cell planes
                     const size_t o = (size_t)k * Nc + g;
-                    if (h->visc) tf_e.push_back(c2n[o]);
                     tf_nx.push_back(gnx[o]);
                     tf_ny.push_back(gny[o]);
                     tf_len.push_back(glen[o]);
@@ -888,8 +881,8 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
     ALLOC(d_dn, Nc); UPLOAD(d_dn, dn);
     ALLOC(d_up, Nc); UPLOAD(d_up, up);
     if (h->quads) { ALLOC(d_dn2, Nc); UPLOAD(d_dn2, dn2); ALLOC(d_up2, Nc); UPLOAD(d_up2, up2); }
-    // (with cn the FP64 kernels read c2n for the analytic ghost state only)
-    if (h->mixed || h->tgv || cn.empty()) { ALLOC(d_c2n, (size_t)nfmax * Nc); UPLOAD(d_c2n, c2n); }
+    // (with cn the kernels read c2n for the analytic ghost state only)
+    if (h->tgv || cn.empty()) { ALLOC(d_c2n, (size_t)nfmax * Nc); UPLOAD(d_c2n, c2n); }
     if (!cn.empty()) {
         int4 *d_cn;
         ALLOC(d_cn, Nc); UPLOAD(d_cn, cn);
@@ -984,11 +977,6 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
         ALLOC(d_tfo, tf_off.size()); UPLOAD(d_tfo, tf_off);
         ALLOC(d_tfr, tf_rec.size()); UPLOAD(d_tfr, tf_rec);
         if (h->quads) { ALLOC(d_tfq, tf_q.size()); UPLOAD(d_tfq, tf_q); }
-        if (h->mixed && h->visc) {
-            int2 *d_tfe;
-            ALLOC(d_tfe, tf_e.size()); UPLOAD(d_tfe, tf_e);
-            m.tf_e = d_tfe;
-        }
         if (h->mixed) {
             // (the FP64 tile kernel reads the face geometry from the per-cell
             // planes, which its viscous source reads too)

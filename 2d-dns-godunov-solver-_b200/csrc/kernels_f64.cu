@@ -64,7 +64,8 @@ cudaError_t launch_visc_grad_f64(const DevMesh &m, const DevState &s, const Laun
     cudaError_t e = (m.nfmax == 4) ? launch_dependent(k_grad1_cells<true>, grid_for(m.Nc, b), b, st, m, s)
                                    : launch_dependent(k_grad1_cells<false>, grid_for(m.Nc, b), b, st, m, s);
     if (e != cudaSuccess) return e;
-    return launch_dependent(k_grad1_nodes, grid_for(m.Nn, b), b, st, m, s);
+    if (m.Nn <= kSplitNodes) return launch_dependent(k_grad1_nodes<1>, grid_for(3 * m.Nn, b), b, st, m, s);
+    return launch_dependent(k_grad1_nodes<3>, grid_for(m.Nn, b), b, st, m, s);
 }
 
 cudaError_t launch_init_state_f64(const DevMesh &m, const DevState &s, int64_t t0, int64_t t1, const LaunchCfg &lc,

@@ -77,8 +77,10 @@ __global__ void __launch_bounds__(256, MINB) k_cell_step_mixed(const DevMesh m, 
                 for (int v = 0; v < 4; ++v) F[v] += f[v];
             }
             float diff[4] = {0.f, 0.f, 0.f, 0.f};
-            if (VISC) diff_source_f<QUAD>(m, s, P, g, is_quad, me, diff);
-            cell_update_mixed(m, s, P, g, me, F, diff, dt, load_cell_in_f(m, s, g), pout, part);
+            if (VISC)
+                diff_source_f<QUAD>(m, s, P, g, is_quad, me, cell_nodes(m, g), ld_once(m.rareaf + g),
+                                    ld_once(m.hxf + g), diff);
+            cell_update_mixed(m, s, P, g, me.x, F, diff, dt, load_cell_in_f(m, s, g), pout, part);
         }
         tile_record<false, false>(m, s, tile, part, s_red);
     }
@@ -167,22 +169,36 @@ __global__ void __launch_bounds__(256, GD2D_NODE_MINB_MIXED) k_grad1_cells_mixed
         const float rA = ld_once(m.rareaf + g);
         float nlx[NF], nly[NF];
         int2 e[NF];
+        const int4 cn = cell_nodes(m, g);
 #pragma unroll
         for (int k = 0; k < NF; ++k) {
             const int64_t o = (int64_t)k * m.Nc + g;
             nlx[k] = ld_once(m.nlxf + o);
             nly[k] = ld_once(m.nlyf + o);
-            e[k] = ld_once(m.c2n + o);
+            if (!m.cn) e[k] = ld_once(m.c2n + o);
         }
         const int nf = (QUAD && ld_once(m.lenf + (int64_t)(NF - 1) * m.Nc + g) != 0.f) ? 4 : 3;
         float sx[3] = {0.f, 0.f, 0.f}, sy[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-        for (int k = 0; k < NF; ++k) {
-            if (k >= nf) break;
-            const float4 A = s.nodeCf[e[k].x], B = s.nodeCf[e[k].y];
+        auto edge = [&](int k, const float4 &A, const float4 &B) {
             sx[0] += 0.5f * (A.x + B.x) * -nly[k]; sy[0] += 0.5f * (A.x + B.x) * -nlx[k];
             sx[1] += 0.5f * (A.y + B.y) * -nly[k]; sy[1] += 0.5f * (A.y + B.y) * -nlx[k];
             sx[2] += 0.5f * (A.z + B.z) * -nly[k]; sy[2] += 0.5f * (A.z + B.z) * -nlx[k];
+        };
+        if (m.cn) {
+            const float4 A = s.nodeCf[cn.x], B = s.nodeCf[cn.y], C = s.nodeCf[cn.z];
+            edge(0, A, B);
+            edge(1, B, C);
+            if (nf == 3) {
+                edge(2, C, A);
+            } else {
+                const float4 D = s.nodeCf[cn.w];
+                edge(2, C, D);
+                edge(NF - 1, D, A);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < NF; ++k)
+                if (k < nf) edge(k, s.nodeCf[e[k].x], s.nodeCf[e[k].y]);
         }
         if (rA == 0.f) continue;
         NodeGradF r;
@@ -193,34 +209,11 @@ __global__ void __launch_bounds__(256, GD2D_NODE_MINB_MIXED) k_grad1_cells_mixed
     }
 }
 
+template <int NV>
 __global__ void __launch_bounds__(256, GD2D_NODE_MINB_MIXED) k_grad1_nodes_mixed(const DevMesh m, const DevState s) {
-    const int W = m.cluster_w;
     pdl_trigger();
     pdl_wait();
-    for (int64_t J = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; J < m.Nn; J += (int64_t)gridDim.x * blockDim.x) {
-        float v[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        int cnt = 0;
-        auto add = [&](const NodeGradF &q) {
-            v[0] += q.ru.x; v[1] += q.ru.y; v[2] += q.rv.x; v[3] += q.rv.y; v[4] += q.re.x; v[5] += q.re.y;
-            ++cnt;
-        };
-        int ci[kMaxCluster];
-#pragma unroll
-        for (int j = 0; j < kMaxCluster; ++j) ci[j] = (j < W) ? ld_once(m.cl + (int64_t)j * m.Nn + J) : -1;
-#pragma unroll
-        for (int j = 0; j < kMaxCluster; ++j)
-            if (ci[j] >= 0) add(s.g1f[ci[j]]);
-        for (int j = kMaxCluster; j < W; ++j) {
-            const int c = ld_once(m.cl + (int64_t)j * m.Nn + J);
-            if (c >= 0) add(s.g1f[c]);
-        }
-        const float r = cnt ? 1.f / (float)cnt : 0.f;
-        NodeGradF o;
-        o.ru = make_float2(v[0] * r, v[1] * r);
-        o.rv = make_float2(v[2] * r, v[3] * r);
-        o.re = make_float2(v[4] * r, v[5] * r);
-        s.nodeGf[J] = o;
-    }
+    grad1_nodes<NV>(m, reinterpret_cast<const float2 *>(s.g1f), reinterpret_cast<float2 *>(s.nodeGf));
 }
 
 // U holds FP64 primitives on entry: conservatives (utilsFVM2dp.jl:4-17) and
@@ -306,7 +299,8 @@ cudaError_t launch_visc_grad_mixed(const DevMesh &m, const DevState &s, const La
     cudaError_t e = (m.nfmax == 4) ? launch_dependent(k_grad1_cells_mixed<true>, grid_for_m(m.Nc, b), b, st, m, s)
                                    : launch_dependent(k_grad1_cells_mixed<false>, grid_for_m(m.Nc, b), b, st, m, s);
     if (e != cudaSuccess) return e;
-    return launch_dependent(k_grad1_nodes_mixed, grid_for_m(m.Nn, b), b, st, m, s);
+    if (m.Nn <= kSplitNodes) return launch_dependent(k_grad1_nodes_mixed<1>, grid_for_m(3 * m.Nn, b), b, st, m, s);
+    return launch_dependent(k_grad1_nodes_mixed<3>, grid_for_m(m.Nn, b), b, st, m, s);
 }
 
 cudaError_t launch_init_state_mixed(const DevMesh &m, const DevState &s, int64_t t0, int64_t t1, const LaunchCfg &lc,

@@ -229,49 +229,53 @@ __device__ __forceinline__ void visc_source_f(const DevCase &P, const float4 &me
     }
 }
 
-// One edge's share of the Green-Gauss sums of the diffusion source, seen
-// from the cell whose inward normal (nx, ny) it has: the first-gradient node
-// means A, B of the edge's two nodes give the Laplacian terms
-// 0.5 (A + B).(-ny, -nx) side of each variable (calcDiffTerm.jl:88-104,
-// gradX paired with -ny), and the node velocities a, b the velocity
-// divergence term 0.5 (a + b).(-nx, -ny) side of the artificial viscosity.
-// The other cell of the edge sees the exact negation.
-__device__ __forceinline__ float4 visc_face_f(const NodeGradF &A, const NodeGradF &B, const float4 &a,
-                                              const float4 &b, float nx, float ny, float side, bool art) {
-    const float cx = -ny * 0.5f * side, cy = -nx * 0.5f * side;
-    float4 r;
-    r.x = (A.ru.x + B.ru.x) * cx + (A.ru.y + B.ru.y) * cy;
-    r.y = (A.rv.x + B.rv.x) * cx + (A.rv.y + B.rv.y) * cy;
-    r.z = (A.re.x + B.re.x) * cx + (A.re.y + B.re.y) * cy;
-    r.w = art ? (a.y + b.y) * cy + (a.z + b.z) * cx : 0.f;
-    return r;
-}
-
-// Diffusion source (calcDiffTerm.jl:88-113 and the extension models) in FP32.
+// Diffusion source (calcDiffTerm.jl:88-113 and the extension models) in FP32:
+// each edge's share of the Green-Gauss sums is 0.5 (A + B).(-ny, -nx) side of
+// its nodes' first-gradient means A, B (gradX paired with -ny) and, for the
+// artificial viscosity's velocity divergence, 0.5 (a + b).(-nx, -ny) side of
+// their velocities.  The edge weights are n * side, rounded once.  cn: the
+// cell's nodes in edge order (DevMesh::cn), each gathered once.
 template <bool QUAD>
 __device__ __forceinline__ void diff_source_f(const DevMesh &m, const DevState &s, const DevCase &P, int64_t g,
-                                              bool is_quad, const float4 &me, float *diff) {
+                                              bool is_quad, const float4 &me, const int4 &cn, float rA, float HX,
+                                              float *diff) {
     const int nf = (QUAD && is_quad) ? 4 : 3;
-    float sx[3] = {0.f, 0.f, 0.f}, sy[3] = {0.f, 0.f, 0.f};
-    float du = 0.f, dv = 0.f;
+    float lap[3] = {0.f, 0.f, 0.f}, div = 0.f;
     const bool art = (P.visc_model != VISC_REFERENCE) && P.art_visc;
-    for (int k = 0; k < nf; ++k) {
+    auto edge = [&](int k, const NodeGradF &A, const NodeGradF &B, const float2 &na, const float2 &nb) {
         const int64_t o = (int64_t)k * m.Nc + g;
-        const float side = ld_once(m.lenf + o), nx = ld_once(m.nxf + o), ny = ld_once(m.nyf + o);
-        const int2 e = ld_once(m.c2n + o);
-        const NodeGradF A = s.nodeGf[e.x], B = s.nodeGf[e.y];
-        sx[0] += 0.5f * (A.ru.x + B.ru.x) * -ny * side; sy[0] += 0.5f * (A.ru.y + B.ru.y) * -nx * side;
-        sx[1] += 0.5f * (A.rv.x + B.rv.x) * -ny * side; sy[1] += 0.5f * (A.rv.y + B.rv.y) * -nx * side;
-        sx[2] += 0.5f * (A.re.x + B.re.x) * -ny * side; sy[2] += 0.5f * (A.re.y + B.re.y) * -nx * side;
-        if (art) {
-            const float4 na = s.nodePf[e.x], nb = s.nodePf[e.y];
-            du += 0.5f * (na.y + nb.y) * -nx * side;
-            dv += 0.5f * (na.z + nb.z) * -ny * side;
+        const float cx = -0.5f * ld_once(m.nlyf + o), cy = -0.5f * ld_once(m.nlxf + o);
+        lap[0] += (A.ru.x + B.ru.x) * cx + (A.ru.y + B.ru.y) * cy;
+        lap[1] += (A.rv.x + B.rv.x) * cx + (A.rv.y + B.rv.y) * cy;
+        lap[2] += (A.re.x + B.re.x) * cx + (A.re.y + B.re.y) * cy;
+        if (art) div += (na.x + nb.x) * cy + (na.y + nb.y) * cx;
+    };
+    auto velocity = [&](int n) {
+        return art ? make_float2(s.nodePf[n].y, s.nodePf[n].z) : make_float2(0.f, 0.f);
+    };
+    if (m.cn) {
+        const NodeGradF A = s.nodeGf[cn.x], B = s.nodeGf[cn.y], C = s.nodeGf[cn.z];
+        const float2 na = velocity(cn.x), nb = velocity(cn.y), nc = velocity(cn.z);
+        edge(0, A, B, na, nb);
+        edge(1, B, C, nb, nc);
+        if (nf == 3) {
+            edge(2, C, A, nc, na);
+        } else {
+            const NodeGradF D = s.nodeGf[cn.w];
+            const float2 nd = velocity(cn.w);
+            edge(2, C, D, nc, nd);
+            edge(3, D, A, nd, na);
+        }
+    } else {
+#pragma unroll 1
+        for (int k = 0; k < nf; ++k) {
+            const int2 e = ld_once(m.c2n + (int64_t)k * m.Nc + g);
+            edge(k, s.nodeGf[e.x], s.nodeGf[e.y], velocity(e.x), velocity(e.y));
         }
     }
-    const float rA = ld_once(m.rareaf + g);
-    const float lap[3] = {(sx[0] + sy[0]) * rA, (sx[1] + sy[1]) * rA, (sx[2] + sy[2]) * rA};
-    visc_source_f(P, me, lap, (du + dv) * rA, art ? ld_once(m.hxf + g) : 0.f, diff);
+#pragma unroll
+    for (int v = 0; v < 3; ++v) lap[v] *= rA;
+    visc_source_f(P, me, lap, div * rA, HX, diff);
 }
 
 // FP32 increment, FP64 accumulation of the Euler update
@@ -294,7 +298,7 @@ __device__ __forceinline__ CellInF load_cell_in_f(const DevMesh &m, const DevSta
 }
 
 __device__ __forceinline__ void cell_update_mixed(const DevMesh &m, const DevState &s, const DevCase &P, int64_t g,
-                                                  const float4 &me, const float *F, const float *diff, double dt,
+                                                  float rho_in, const float *F, const float *diff, double dt,
                                                   const CellInF &in, float4 *__restrict__ pout, Part &part) {
     const float bdt = (float)(P.beta * dt);
     const double4 U = in.U;
@@ -309,7 +313,7 @@ __device__ __forceinline__ void cell_update_mixed(const DevMesh &m, const DevSta
     }
     st_once(s.U + g, make_double4(Un[0], Un[1], Un[2], Un[3]));
     const double rho = Un[0];
-    const double rinv = 1.0 / rho;
+    const double rinv = rcp_rn(rho);  // a state outside its range is a failed one
     const double ux = Un[1] * rinv;
     const double uy = Un[2] * rinv;
     const double p = (P.gamma - 1.0) * (Un[3] - 0.5 * (Un[1] * ux + Un[2] * uy));
@@ -326,8 +330,8 @@ __device__ __forceinline__ void cell_update_mixed(const DevMesh &m, const DevSta
     part.ek = 0.5 * rho * (ux * ux + uy * uy) * area;
     part.vmax = (double)vmax;
     part.rmin = (double)(in.charlen / vmax);
-    part.rhomin = (double)me.x;
-    part.rhomax = (double)me.x;
+    part.rhomin = (double)rho_in;
+    part.rhomax = (double)rho_in;
     const bool ok = isfinite(Un[0]) && isfinite(Un[1]) && isfinite(Un[2]) && isfinite(Un[3]) && (rho > 0.0) &&
                     (p > 0.0);
     part.bad = ok ? 0.0 : 1.0;

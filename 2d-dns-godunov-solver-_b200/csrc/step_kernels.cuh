@@ -882,30 +882,43 @@ __global__ void __launch_bounds__(256, GD2D_NODE_MINB) k_node_avg(const DevMesh 
     const int W = m.cluster_w;
     for (int64_t J = n0 + bid * blockDim.x + threadIdx.x; J < n1; J += nblk * blockDim.x) {
         bool prim_form = false;
-        double gop = 0.0, gam = 0.0;
+        double gop = 0.0, gm1 = 0.0;
         if (VISC) {
             const DevCase &P = m.cases[ld_once(m.node_case + J)];
             prim_form = P.visc_model != VISC_REFERENCE;
             gop = P.gamma_over_Pr;
-            gam = P.gamma;
+            gm1 = P.face.gm1;
         }
         double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0, det = 0.0;
         double c0 = 0.0, c1 = 0.0, c2 = 0.0;
         int cnt = 0;
+        // phi = |u|^2/2 + (gamma/Pr) p / ((gamma-1) rho)
+        auto phi_plain = [&](const double4 &p) {
+            return 0.5 * (p.y * p.y + p.z * p.z) + gop * (p.w / (gm1 * p.x));
+        };
+        Divisors<-150, 200> dr(1.0);
+        InRange<-150, 200> pr(1.0);
         auto add = [&](int c, const double4 &p, double w) {
-            a0 = a0 + p.x * w; a1 = a1 + p.y * w; a2 = a2 + p.z * w; a3 = a3 + p.w * w;
-            det = det + w;
+            if (UNIT) {
+                a0 = a0 + p.x; a1 = a1 + p.y; a2 = a2 + p.z; a3 = a3 + p.w;
+            } else {
+                a0 = a0 + p.x * w; a1 = a1 + p.y * w; a2 = a2 + p.z * w; a3 = a3 + p.w * w;
+                det = det + w;
+            }
             if (VISC) {
                 if (prim_form) {
-                    // u, v, phi = |u|^2/2 + (gamma/Pr) p / ((gamma-1) rho)
-                    const double ph = 0.5 * (p.y * p.y + p.z * p.z) + gop * (p.w / ((gam - 1.0) * p.x));
-                    c0 = c0 + p.y; c1 = c1 + p.z; c2 = c2 + ph;
+                    // (unit weights: the velocities' means are the primitives')
+                    if (!UNIT) { c0 = c0 + p.y; c1 = c1 + p.z; }
+                    const double d = gm1 * p.x;
+                    dr.add(d);
+                    pr.add(p.w);
+                    c2 = c2 + (0.5 * (p.y * p.y + p.z * p.z) + gop * div_rn(p.w, d));
                 } else {
                     const double4 u = s.U[c];
                     c0 = c0 + u.y; c1 = c1 + u.z; c2 = c2 + u.w;
                 }
-                ++cnt;
             }
+            ++cnt;
         };
         // all cluster indices first, then the gathers in an unrolled
         // sequence the compiler can overlap (sums keep the reference order)
@@ -919,15 +932,38 @@ __global__ void __launch_bounds__(256, GD2D_NODE_MINB) k_node_avg(const DevMesh 
             const int c = ld_once(m.cl + (int64_t)j * m.Nn + J);
             if (c >= 0) add(c, src[c], UNIT ? 1.0 : ld_once(m.wt + (int64_t)j * m.Nn + J));
         }
-        if (det != 0.0) { a0 = a0 / det; a1 = a1 / det; a2 = a2 / det; a3 = a3 / det; }
+        if (VISC && prim_form && __builtin_expect(!(dr.ok() && pr.ok()), 0)) {
+            c2 = 0.0;
+            for (int j = 0; j < W; ++j) {
+                const int c = m.cl[(int64_t)j * m.Nn + J];
+                if (c >= 0) c2 = c2 + phi_plain(src[c]);
+            }
+        }
+        if (UNIT) det = (double)cnt;
+        // quotients over the count share its reciprocal (unit weights; sums
+        // too small for that, and other weights, take the plain `/`)
+        const double dc = (double)cnt, y = rcp_rn(dc);
+        Numerators tiny(a0);
+        tiny.add(a1); tiny.add(a2); tiny.add(a3);
+        if (VISC) { tiny.add(c0); tiny.add(c1); tiny.add(c2); }
+        const double huge = fmax(fmax(fabs(a0), fabs(a1)), fmax(fabs(a2), fabs(a3)));
+        const bool finite = huge < 1e200 && (!VISC || (fabs(c0) < 1e200 && fabs(c1) < 1e200 && fabs(c2) < 1e200)) &&
+                            !(a0 != a0 || a1 != a1 || a2 != a2 || a3 != a3);
+        const bool exact = cnt != 0 && finite && tiny.ok();
+        if (UNIT && exact) {
+            a0 = div_by(a0, dc, y); a1 = div_by(a1, dc, y); a2 = div_by(a2, dc, y); a3 = div_by(a3, dc, y);
+        } else if (det != 0.0) {
+            a0 = a0 / det; a1 = a1 / det; a2 = a2 / det; a3 = a3 / det;
+        }
         s.nodeP[J] = zero_prims ? make_double4(0.0, 0.0, 0.0, 0.0) : make_double4(a0, a1, a2, a3);
         if (VISC) {
-            if (cnt != 0) {
-                const double dc = (double)cnt;
-                s.nodeC[J] = make_double4(c0 / dc, c1 / dc, c2 / dc, 0.0);
-            } else {
-                s.nodeC[J] = make_double4(0.0, 0.0, 0.0, 0.0);
+            if (exact) {
+                c0 = div_by(c0, dc, y); c1 = div_by(c1, dc, y); c2 = div_by(c2, dc, y);
+            } else if (cnt != 0) {
+                c0 = c0 / dc; c1 = c1 / dc; c2 = c2 / dc;
             }
+            if (UNIT && prim_form) { c0 = a1; c1 = a2; }
+            s.nodeC[J] = make_double4(c0, c1, c2, 0.0);
         }
     }
     if (flip) {
@@ -1027,17 +1063,29 @@ __global__ void __launch_bounds__(256, GD2D_NODE_MINB) k_grad1_cells(const DevMe
 }
 
 // Unweighted node means of the first gradients (calcPhiInCellCluster on the
-// gradient fields, calcGradients.jl:3-18).
-static __global__ void __launch_bounds__(256, GD2D_NODE_MINB) k_grad1_nodes(const DevMesh m, const DevState s) {
+// gradient fields, calcGradients.jl:3-18), bound by the latency of their
+// gathers.  NV = 3: one thread a node takes its three variables in turn.
+// NV = 1: three neighbouring threads a node take one variable each, 16 (mixed:
+// 8) bytes of a gather's 48 (24), which puts three times the threads to work
+// on a mesh that does not fill the device but reads the cluster lists three
+// times.  T2: double2 or float2.
+template <int NV, class T2>
+__device__ __forceinline__ void grad1_nodes(const DevMesh &m, const T2 *__restrict__ g1, T2 *__restrict__ out) {
     const int W = m.cluster_w;
-    pdl_trigger();
-    pdl_wait();
-    for (int64_t J = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; J < m.Nn; J += (int64_t)gridDim.x * blockDim.x) {
-        double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (3 / NV) * m.Nn;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t J = NV == 3 ? i : (int64_t)((unsigned)i / 3u), v0 = NV == 3 ? 0 : i - 3 * J;
+        T2 x[NV];
+#pragma unroll
+        for (int v = 0; v < NV; ++v) x[v].x = x[v].y = 0;
         int cnt = 0;
-        auto add = [&](const NodeGrad &q) {
-            v[0] = v[0] + q.ru.x; v[1] = v[1] + q.ru.y; v[2] = v[2] + q.rv.x;
-            v[3] = v[3] + q.rv.y; v[4] = v[4] + q.re.x; v[5] = v[5] + q.re.y;
+        auto add = [&](int64_t c) {
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                const T2 q = g1[3 * c + v0 + v];
+                x[v].x = x[v].x + q.x;
+                x[v].y = x[v].y + q.y;
+            }
             ++cnt;
         };
         int ci[kMaxCluster];
@@ -1045,22 +1093,27 @@ static __global__ void __launch_bounds__(256, GD2D_NODE_MINB) k_grad1_nodes(cons
         for (int j = 0; j < kMaxCluster; ++j) ci[j] = (j < W) ? ld_once(m.cl + (int64_t)j * m.Nn + J) : -1;
 #pragma unroll
         for (int j = 0; j < kMaxCluster; ++j)
-            if (ci[j] >= 0) add(s.g1[ci[j]]);
+            if (ci[j] >= 0) add(ci[j]);
         for (int j = kMaxCluster; j < W; ++j) {
             const int c = ld_once(m.cl + (int64_t)j * m.Nn + J);
-            if (c >= 0) add(s.g1[c]);
+            if (c >= 0) add(c);
         }
-        NodeGrad r;
-        if (cnt != 0) {
-            const double dc = (double)cnt;
-            r.ru = make_double2(v[0] / dc, v[1] / dc);
-            r.rv = make_double2(v[2] / dc, v[3] / dc);
-            r.re = make_double2(v[4] / dc, v[5] / dc);
-        } else {
-            r.ru = r.rv = r.re = make_double2(0.0, 0.0);
+        using T = decltype(x[0].x);
+        const T dc = cnt != 0 ? cnt : 1;  // (the sums of no cells are zero)
+        const T r = T(1) / dc;            // FP32 multiplies by the reciprocal
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            x[v].x = sizeof(T) == 4 ? x[v].x * r : x[v].x / dc;
+            x[v].y = sizeof(T) == 4 ? x[v].y * r : x[v].y / dc;
+            out[3 * J + v0 + v] = x[v];
         }
-        s.nodeG[J] = r;
     }
+}
+template <int NV>
+__global__ void __launch_bounds__(256, GD2D_NODE_MINB) k_grad1_nodes(const DevMesh m, const DevState s) {
+    pdl_trigger();
+    pdl_wait();
+    grad1_nodes<NV>(m, reinterpret_cast<const double2 *>(s.g1), reinterpret_cast<double2 *>(s.nodeG));
 }
 
 // ------------------------------------------------------------ state init
