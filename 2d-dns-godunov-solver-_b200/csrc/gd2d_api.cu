@@ -456,9 +456,11 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
         return fail(nullptr, GD2D_ERR_ARG, "block must be 128 or 256");
     }
     h->lc.block = block;
-    // node-side passes: 64-thread blocks measured fastest (finer-grained
-    // scheduling of their gathers; 2% of the step on the 2.09M-cell cylinder)
-    h->lc.node_block = h->launch.node_block ? h->launch.node_block : 64;
+    // node-side passes: 128-thread blocks, four warps for the fold of a small
+    // case.  us a step, 64 / 128 / 256: 2,048 cells 17.3 / 16.4 / 15.4, 36,000
+    // mixed 13.5 / 11.7 / 11.3, 523,000 mixed 67.2 / 65.3 / 65.7, 2.09M FP64
+    // 407 / 409 / 416
+    h->lc.node_block = h->launch.node_block ? h->launch.node_block : 128;
     if (h->lc.node_block != 64 && h->lc.node_block != 128 && h->lc.node_block != 256) {
         delete h;
         return fail(nullptr, GD2D_ERR_ARG, "node_block must be 64, 128 or 256");

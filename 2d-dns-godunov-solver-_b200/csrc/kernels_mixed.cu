@@ -92,11 +92,13 @@ template <bool VISC, bool UNIT>
 __global__ void __launch_bounds__(256, GD2D_NODE_MINB_MIXED) k_node_avg_mixed(const DevMesh m, const DevState s, int flip, int zero_prims,
                                                         int64_t n0, int64_t n1, int64_t g0, int nred, int is_init) {
     pdl_trigger();
-    pdl_wait();
     if ((int)blockIdx.x < nred) {
-        fold_block<false>(m, s, g0, is_init != 0);
+        const FoldTask task = fold_task(m, g0);
+        pdl_wait();
+        fold_block<false>(m, s, task, is_init != 0);
         return;
     }
+    pdl_wait();
     const int64_t bid = (int64_t)blockIdx.x - nred, nblk = (int64_t)gridDim.x - nred;
     const int par = *s.parity;
     const float4 *__restrict__ src = s.primf + (int64_t)(flip ? (par ^ 1) : par) * m.Nc;

@@ -126,47 +126,45 @@ __device__ __forceinline__ Part warp_reduce_records(const double *recs, int64_t 
     return acc;
 }
 
-// Per-case finalization by the warp that completed the case's last tile
-// group: reduce the group records in a fixed order, publish the step
-// statistics and advance time (flowTime += dt, testInviscidFluxesGPUx32.jl:401)
+// Per-case finalization, by one thread, from the case's reduction and its
+// state `in` before the step: publish the step statistics and advance time (flowTime += dt, testInviscidFluxesGPUx32.jl:401)
 // and the next dt: the fixed solControls.dt the reference steps with, or
 // opt-in, the tau it reports (testInviscidFluxesGPUx32.jl:299,324) or the
 // local-CFL extension.
-static __device__ __forceinline__ void finalize_case(const DevMesh &m, const DevState &s, int c, bool is_init) {
+static __device__ __forceinline__ void finalize_case(const DevMesh &m, const DevState &s, int c, const CaseState &in,
+                                                     const Part &acc, bool is_init) {
     const DevCase &P = m.cases[c];
-    const Part acc = warp_reduce_records(s.gpart, P.group_begin, P.group_end);
-    if ((threadIdx.x & 31) == 0) {
-        CaseState *cs = s.cstate + c;
-        double vnew = acc.vmax, rnew = acc.rmin;
-        if (!is_init) {
-            DevStats st;
-            st.dt = cs->dt;
-            st.flow_time = cs->t;
-            st.velmax = cs->velmax;
-            st.tau = P.CFL * P.maxEdge / jl_max(cs->velmax, 1.0e-6);
-            for (int v = 0; v < 4; ++v) { st.residual[v] = acc.res[v]; st.totals[v] = acc.tot[v]; }
-            st.rho_min = acc.rhomin;
-            st.rho_max = acc.rhomax;
-            st.kinetic_energy = acc.ek;
-            st.step = cs->step + 1;
-            st.nonfinite = acc.bad > 0.0 ? 1 : 0;
-            st.reserved0 = 0;
-            const int64_t row = (cs->step % s.ring_len) * m.ncases + c;
-            s.ring[row] = st;
-            s.ring_host[row] = st;  // over PCIe: the host reads it after the stream's sync
-            cs->t = cs->t + cs->dt;
-            cs->step = cs->step + 1;
-            if (acc.bad > 0.0) cs->nonfinite = 1;
-        }
-        double dtn;
-        if (P.dt_mode == DT_REFERENCE_TAU) dtn = P.CFL * P.maxEdge / jl_max(vnew, 1.0e-6);
-        else if (P.dt_mode == DT_LOCAL_CFL) dtn = P.CFL * rnew;
-        else dtn = P.dt_fixed;
-        cs->dt = dtn;
-        cs->velmax = vnew;
-        cs->rmin = rnew;
-        cs->tiles_done = 0u;
+    CaseState out = in;
+    const double vnew = acc.vmax, rnew = acc.rmin;
+    if (!is_init) {
+        DevStats st;
+        st.dt = in.dt;
+        st.flow_time = in.t;
+        st.velmax = in.velmax;
+        st.tau = P.CFL * P.maxEdge / jl_max(in.velmax, 1.0e-6);
+        for (int v = 0; v < 4; ++v) { st.residual[v] = acc.res[v]; st.totals[v] = acc.tot[v]; }
+        st.rho_min = acc.rhomin;
+        st.rho_max = acc.rhomax;
+        st.kinetic_energy = acc.ek;
+        st.step = in.step + 1;
+        st.nonfinite = acc.bad > 0.0 ? 1 : 0;
+        st.reserved0 = 0;
+        const int64_t row = (in.step % s.ring_len) * m.ncases + c;
+        s.ring[row] = st;
+        s.ring_host[row] = st;  // over PCIe: the host reads it after the stream's sync
+        out.t = in.t + in.dt;
+        out.step = in.step + 1;
+        if (acc.bad > 0.0) out.nonfinite = 1;
     }
+    double dtn;
+    if (P.dt_mode == DT_REFERENCE_TAU) dtn = P.CFL * P.maxEdge / jl_max(vnew, 1.0e-6);
+    else if (P.dt_mode == DT_LOCAL_CFL) dtn = P.CFL * rnew;
+    else dtn = P.dt_fixed;
+    out.dt = dtn;
+    out.velmax = vnew;
+    out.rmin = rnew;
+    out.tiles_done = 0u;
+    s.cstate[c] = out;
 }
 
 // Field f of tile q's reduction record.  Two layouts, measured per
@@ -275,54 +273,98 @@ __host__ __device__ __forceinline__ int fold_blocks_per_group(int block) {
     return (kPartFields + nw - 1) / nw;
 }
 
-// The step's two-level reduction, done by warps of the node pass that
-// follows the cell kernel (the cell kernel's tile records are visible
-// there: pdl_wait has returned).  One warp folds field f of tile group
-// `gid` (up to kGroupTiles tiles of one case) into the group's record: lane
-// l takes records l, l + 32, ..., l + kGroupTiles - 32 of the group in
-// turn, then a fixed shuffle tree over the lanes.  It then counts the field
-// done for the case; the warp that completes the case's last (group, field)
-// pair reduces the case's group records and finalizes the case
-// (finalize_case).  No thread waits on another's atomic; whichever warp
-// finalizes, the order of every sum is the same, so the results are
-// deterministic and do not depend on the node pass's block size.
+// The step's two-level reduction, done by the first blocks of the node pass
+// that follows the cell kernel (the cell kernel's tile records are visible
+// there: pdl_wait has returned).  A warp folds one field of one tile group
+// (up to kGroupTiles tiles of one case): lane l takes records l, l + 32, ...,
+// l + kGroupTiles - 32 of the group in turn, then a fixed shuffle tree over
+// the lanes.  No thread waits on another's atomic and no order depends on
+// which warp finishes last or on the node pass's block size, so the results
+// are deterministic.
+//
+// What is known before the wait: the block's group and case.
+struct FoldTask {
+    int c, n;        // case; tiles of the group
+    int64_t gid, t0; // group; its first tile
+    int groups;      // groups of the case
+};
+__device__ __forceinline__ FoldTask fold_task(const DevMesh &m, int64_t g0) {
+    FoldTask k;
+    k.gid = g0 + blockIdx.x / fold_blocks_per_group(blockDim.x);
+    k.c = m.group_case[k.gid];
+    const DevCase &P = m.cases[k.c];
+    k.t0 = P.tile_begin + (k.gid - P.group_begin) * kGroupTiles;
+    k.n = (int)((k.t0 + kGroupTiles < P.tile_end) ? kGroupTiles : P.tile_end - k.t0);
+    k.groups = (int)(P.group_end - P.group_begin);
+    return k;
+}
 template <bool FIELD_MAJOR>
-static __device__ __forceinline__ void fold_field(const DevMesh &m, const DevState &s, int64_t gid, int f,
-                                               bool is_init) {
+__device__ __forceinline__ double fold_group(const DevMesh &m, const DevState &s, const FoldTask &k, int f) {
     constexpr int kPerLane = kGroupTiles / 32;
-    const int c = m.group_case[gid];
-    const DevCase &P = m.cases[c];
-    const int64_t t0 = P.tile_begin + (gid - P.group_begin) * kGroupTiles;
-    const int n = (int)((t0 + kGroupTiles < P.tile_end) ? kGroupTiles : P.tile_end - t0);
     const int lane = threadIdx.x & 31;
     const double id = part_ident(f);
     double v[kPerLane];
 #pragma unroll
-    for (int j = 0; j < kPerLane; ++j) v[j] = (lane + 32 * j < n) ? __ldcg(part_at<FIELD_MAJOR>(m, s, t0 + lane + 32 * j, f)) : id;
+    for (int j = 0; j < kPerLane; ++j)
+        v[j] = (lane + 32 * j < k.n) ? __ldcg(part_at<FIELD_MAJOR>(m, s, k.t0 + lane + 32 * j, f)) : id;
     double x = v[0];
 #pragma unroll
     for (int j = 1; j < kPerLane; ++j) x = part_op(f, x, v[j]);
     for (int off = 16; off > 0; off >>= 1) x = part_op(f, x, __shfl_down_sync(0xffffffffu, x, off));
+    return x;
+}
+
+// Block b < nred of a node pass.  A case of one group (up to 65,536 cells) is
+// folded and finalized by one block of four or more warps through shared
+// memory (two warps would take seven fields in turn).  Otherwise a warp
+// takes one (group, field) pair, writes it to the group's record and counts
+// it done for the case; the warp that completes the case's last pair reduces
+// the case's group records and finalizes the case.  On a small mesh the fold
+// is the step's critical path: eight dependent trips to memory through the
+// records, fences and the counter made the step 2.4 us longer than without
+// (7,900-cell Taylor-Green box 20.2 us a step, by one block 16.3).
+template <bool FIELD_MAJOR>
+__device__ __forceinline__ void fold_block(const DevMesh &m, const DevState &s, const FoldTask &k, bool is_init) {
+    __shared__ double s_fold[kPartials];
+    const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5, part = blockIdx.x % fold_blocks_per_group(blockDim.x);
+    const int lane = threadIdx.x & 31;
+    if (k.groups == 1 && nw >= 4) {
+        if (part != 0) return;
+        CaseState in = {};
+        if (threadIdx.x == 0) in = s.cstate[k.c];
+        for (int f = warp; f < kPartFields; f += nw) {
+            const double x = fold_group<FIELD_MAJOR>(m, s, k, f);
+            if (lane == 0) s_fold[f] = x;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            Part acc;
+            acc.init();
+            Part o;
+#pragma unroll
+            for (int f = 0; f < kPartFields; ++f) part_set(o, f, s_fold[f]);
+            acc.combine(o);
+            finalize_case(m, s, k.c, in, acc, is_init);
+        }
+        return;
+    }
+    const int f = part * nw + warp;
+    if (f >= kPartFields) return;
+    const double x = fold_group<FIELD_MAJOR>(m, s, k, f);
     int last = 0;
     if (lane == 0) {
-        s.gpart[gid * kPartials + f] = x;  // field f is record slot f
+        s.gpart[k.gid * kPartials + f] = x;  // field f is record slot f
         __threadfence();
-        const unsigned int need = (unsigned int)((P.group_end - P.group_begin) * kPartFields);
-        last = (atomicAdd(&s.cstate[c].tiles_done, 1u) == need - 1u) ? 1 : 0;
+        const unsigned int need = (unsigned int)(k.groups * kPartFields);
+        last = (atomicAdd(&s.cstate[k.c].tiles_done, 1u) == need - 1u) ? 1 : 0;
     }
     last = __shfl_sync(0xffffffffu, last, 0);
     if (last) {
         __threadfence();
-        finalize_case(m, s, c, is_init);
+        const int64_t g = m.cases[k.c].group_begin;
+        const Part acc = warp_reduce_records(s.gpart, g, g + k.groups);
+        if (lane == 0) finalize_case(m, s, k.c, s.cstate[k.c], acc, is_init);
     }
-}
-
-// Block b < nred of a node pass: its warps fold (group, field) pairs.
-template <bool FIELD_MAJOR>
-__device__ __forceinline__ void fold_block(const DevMesh &m, const DevState &s, int64_t g0, bool is_init) {
-    const int bpg = fold_blocks_per_group(blockDim.x);
-    const int f = (int)(blockIdx.x % bpg) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (f < kPartFields) fold_field<FIELD_MAJOR>(m, s, g0 + blockIdx.x / bpg, f, is_init);
 }
 
 // --------------------------------------------------------- MUSCL + flux
@@ -871,11 +913,13 @@ template <bool VISC, bool UNIT>
 __global__ void __launch_bounds__(256, GD2D_NODE_MINB) k_node_avg(const DevMesh m, const DevState s, int flip, int zero_prims,
                                                   int64_t n0, int64_t n1, int64_t g0, int nred, int is_init) {
     pdl_trigger();
-    pdl_wait();
     if ((int)blockIdx.x < nred) {
-        fold_block<true>(m, s, g0, is_init != 0);
+        const FoldTask task = fold_task(m, g0);
+        pdl_wait();
+        fold_block<true>(m, s, task, is_init != 0);
         return;
     }
+    pdl_wait();
     const int64_t bid = (int64_t)blockIdx.x - nred, nblk = (int64_t)gridDim.x - nred;
     const int par = *s.parity;
     const double4 *__restrict__ src = s.prim + (int64_t)(flip ? (par ^ 1) : par) * m.Nc;
