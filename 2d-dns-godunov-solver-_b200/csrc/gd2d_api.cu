@@ -467,8 +467,8 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
     }
     h->lc.persistent = h->launch.persistent;
     // register budget of the cell kernel, measured best on the 2.09M-cell
-    // viscous cylinder: 3 blocks/SM for the FP64 kernels (the tile loop of a
-    // small mesh: see below), 4 for the mixed kernels
+    // viscous cylinder: 3 blocks/SM for the FP64 kernels (small meshes: see
+    // below), 4 for the mixed kernels
     h->lc.min_blocks = h->launch.min_blocks ? h->launch.min_blocks : (h->mixed ? 4 : 3);
     if (h->lc.min_blocks < 2 || h->lc.min_blocks > 4) {
         delete h;
@@ -1035,13 +1035,14 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
     {
         int dev_sms = 148;
         cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, h->device);
-        if (!h->launch.min_blocks && !h->mixed && h->loop == GD2D_LOOP_TILE_FACES) {
-            // FP64 tile loop: the 2-block budget (no spills, a tile in less
+        if (!h->launch.min_blocks && !h->mixed) {
+            // FP64 loops: the 2-block budget (no spills, a tile in less
             // time) where it takes no more waves of blocks than the 3-block
             // one.  us a step, 2 / 3 blocks: square 80 tiles 17.1 / 17.9,
-            // Taylor-Green 512 36.8 / 38.3, Roe square 556 37.0 / 41.9; more
-            // waves: quads 352 51.0 / 47.4, square 704 33.8 / 32.7, cylinder
-            // 2044 123 / 116, 8172 440 / 411
+            // Taylor-Green 512 36.8 / 38.3, Roe square 556 37.0 / 41.9, cell
+            // loop 512 39.6 / 43.8; more waves: quads 352 51.0 / 47.4, square
+            // 704 33.8 / 32.7, cylinder 2044 123 / 116, 8172 440 / 411, cell
+            // loop 8172 479 / 475
             const int64_t per = dev_sms * (256 / block), w2 = (ntiles + 2 * per - 1) / (2 * per);
             h->lc.min_blocks = w2 <= (ntiles + 3 * per - 1) / (3 * per) ? 2 : 3;
         }

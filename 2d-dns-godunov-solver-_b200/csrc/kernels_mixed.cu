@@ -21,6 +21,8 @@ namespace {
 template <int FLUX, bool VISC, bool QUAD, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_cell_step_mixed(const DevMesh m, const DevState s) {
     __shared__ double s_red[8 * kPartials];
+    pdl_trigger();
+    pdl_wait();
     const int par = *s.parity;
     const float4 *__restrict__ pin = s.primf + (int64_t)par * m.Nc;
     float4 *__restrict__ pout = s.primf + (int64_t)(par ^ 1) * m.Nc;
@@ -256,10 +258,9 @@ int grid_for_m(int64_t work, int block) {
 template <int FLUX, bool VISC, bool QUAD>
 cudaError_t cell_step_m(const DevMesh &m, const DevState &s, const LaunchCfg &lc, cudaStream_t st) {
     int grid = lc.persistent ? lc.grid : (int)m.ntiles;
-    if (lc.min_blocks >= 4) k_cell_step_mixed<FLUX, VISC, QUAD, 4><<<grid, lc.block, 0, st>>>(m, s);
-    else if (lc.min_blocks == 3) k_cell_step_mixed<FLUX, VISC, QUAD, 3><<<grid, lc.block, 0, st>>>(m, s);
-    else k_cell_step_mixed<FLUX, VISC, QUAD, 2><<<grid, lc.block, 0, st>>>(m, s);
-    return cudaGetLastError();
+    if (lc.min_blocks >= 4) return launch_dependent(k_cell_step_mixed<FLUX, VISC, QUAD, 4>, grid, lc.block, st, m, s);
+    if (lc.min_blocks == 3) return launch_dependent(k_cell_step_mixed<FLUX, VISC, QUAD, 3>, grid, lc.block, st, m, s);
+    return launch_dependent(k_cell_step_mixed<FLUX, VISC, QUAD, 2>, grid, lc.block, st, m, s);
 }
 
 template <int FLUX>

@@ -741,6 +741,8 @@ __device__ __forceinline__ void cell_update(const DevMesh &m, const DevState &s,
 template <int FLUX, bool VISC, bool QUAD, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_cell_step(const DevMesh m, const DevState s) {
     __shared__ double s_red[8 * kPartials];
+    pdl_trigger();
+    pdl_wait();
     const int par = *s.parity;
     const double4 *__restrict__ pin = s.prim + (int64_t)par * m.Nc;
     double4 *__restrict__ pout = s.prim + (int64_t)(par ^ 1) * m.Nc;
