@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <condition_variable>
 #include <cstdarg>
@@ -18,6 +19,8 @@
 #include <numeric>
 #include <string>
 #include <thread>
+#include <system_error>
+#include <utility>
 #include <vector>
 
 #include "../../include/godunov2d.h"
@@ -199,6 +202,30 @@ int fail(gd2d_handle *h, int code, const char *fmt, ...) {
 
 inline int64_t cidx(int64_t n, int64_t i, int64_t j) { return i + j * n; }
 
+// fn(begin, end) over [0, n) on up to 8 host threads, for the set-up's loops
+// over cells and nodes (gathers from the reference's columns, a cache miss
+// each: on one thread they were half of a 2.09M-cell set-up's 0.95 s).
+// Short loops stay on the calling thread, as does everything if no thread
+// can be started.
+template <class Fn>
+void parallel_ranges(int64_t n, const Fn &fn) {
+    const int64_t least = 1 << 15;
+    const int64_t nt = std::min<int64_t>({8, (int64_t)std::max(1u, std::thread::hardware_concurrency()), n / least});
+    if (nt <= 1) return fn((int64_t)0, n);
+    std::vector<std::thread> th;
+    int64_t begin = 0;
+    try {
+        for (int64_t t = 0; t + 1 < nt; ++t) {
+            const int64_t end = n * (t + 1) / nt;
+            th.emplace_back([&fn, begin, end] { fn(begin, end); });
+            begin = end;
+        }
+    } catch (const std::system_error &) {
+    }
+    fn(begin, n);
+    for (auto &t : th) t.join();
+}
+
 // Hilbert index of (x, y) on a 2^16 grid (Butz / Lam-Shapiro iterative form).
 uint64_t hilbert_index(uint32_t x, uint32_t y) {
     const uint32_t n = 1u << 16;
@@ -227,15 +254,31 @@ void hilbert_order(const std::vector<double> &xs, const std::vector<double> &ys,
     }
     double span = std::max(x1 - x0, y1 - y0);
     if (!(span > 0)) span = 1.0;
-    std::vector<uint64_t> key(n);
-    for (size_t i = 0; i < n; ++i) {
-        uint32_t qx = (uint32_t)std::min(65535.0, std::floor((xs[i] - x0) / span * 65535.0));
-        uint32_t qy = (uint32_t)std::min(65535.0, std::floor((ys[i] - y0) / span * 65535.0));
-        key[i] = hilbert_index(qx, qy);
+    // (index, key) in order of the key, equal keys in order of the index: a
+    // byte-wise radix sort of the 32-bit keys, each pass stable
+    std::vector<std::pair<uint32_t, uint32_t>> a(n), b(n);
+    parallel_ranges((int64_t)n, [&](int64_t b0, int64_t b1) {
+        for (int64_t i = b0; i < b1; ++i) {
+            uint32_t qx = (uint32_t)std::min(65535.0, std::floor((xs[i] - x0) / span * 65535.0));
+            uint32_t qy = (uint32_t)std::min(65535.0, std::floor((ys[i] - y0) / span * 65535.0));
+            a[i] = {(uint32_t)i, (uint32_t)hilbert_index(qx, qy)};
+        }
+    });
+    size_t count[4][256] = {};
+    for (const auto &e : a)
+        for (int d = 0; d < 4; ++d) ++count[d][(e.second >> (8 * d)) & 255u];
+    for (int d = 0; d < 4; ++d) {
+        size_t at = 0;
+        for (size_t &c : count[d]) {
+            const size_t k = c;
+            c = at;
+            at += k;
+        }
+        for (const auto &e : a) b[count[d][(e.second >> (8 * d)) & 255u]++] = e;
+        a.swap(b);
     }
     perm.resize(n);
-    std::iota(perm.begin(), perm.end(), 0);
-    std::stable_sort(perm.begin(), perm.end(), [&](int64_t a, int64_t b) { return key[a] < key[b]; });
+    for (size_t i = 0; i < n; ++i) perm[i] = a[i].first;
 }
 
 // Reverse Cuthill-McKee over the face-neighbour graph of the cells.
@@ -609,6 +652,13 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
     if (h->tgv) { mid.assign(Nc, make_double2(0.0, 0.0)); xnode.assign(Nn, 0.0); ynode.assign(Nn, 0.0); }
     for (int64_t g = 0; g < Nc; ++g) nbr[g] = make_int4(kAbsent, kAbsent, kAbsent, kAbsent);
     for (int64_t g = 0; g < Nc; ++g) { dn[g] = make_int4(0, 0, 0, 0); up[g] = make_int4(0, 0, 0, 0); }
+    // each cell's nodes in edge order, if the edges of every cell are a
+    // closed walk in face order (as the reference's meshes list them): the
+    // gradient passes then gather a node once instead of once per edge.  An
+    // edge's two nodes enter symmetrically, so they may be listed either way.
+    std::vector<int4> cn;
+    std::atomic<bool> closed(h->visc);
+    if (closed) cn.assign(Nc, make_int4(0, 0, 0, 0));
     std::vector<int32_t> tile_case(ntiles, 0);
     std::vector<int32_t> node_case(Nn, 0);
     h->hcases.resize(n_cases);
@@ -623,60 +673,81 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
             if (id1 < 1) return 0;
             return (int32_t)(hc.node_off + hc.node_inv[id1 - 1]);
         };
-        for (int64_t j = 0; j < n; ++j) {
-            const int64_t i = hc.cell_perm[j];
-            const int64_t g = hc.cell_off + j;
-            const int nf = mv.mesh_connectivity[cidx(n, i, 2)];
-            int nb[4] = {kAbsent, kAbsent, kAbsent, kAbsent};
-            int d1[4] = {0, 0, 0, 0}, u1[4] = {0, 0, 0, 0}, d2[4] = {0, 0, 0, 0}, u2[4] = {0, 0, 0, 0};
-            double per = 0.0;
-            for (int k = 0; k < nf; ++k) {
-                int32_t st = mv.cell_stiffness[cidx(n, i, k)];
-                if (st >= 1) {
-                    nb[k] = (int32_t)(hc.cell_off + hc.cell_inv[st - 1]);
-                    d1[k] = node_g(mv.node2cellL2down[cidx(n, i, 2 * k)]);
-                    u1[k] = node_g(mv.node2cellL2up[cidx(n, i, 2 * k)]);
-                    if (nf == 4) {
-                        d2[k] = node_g(mv.node2cellL2down[cidx(n, i, 2 * k + 1)]);
-                        u2[k] = node_g(mv.node2cellL2up[cidx(n, i, 2 * k + 1)]);
+        parallel_ranges(n, [&](int64_t j0, int64_t j1) {
+            for (int64_t j = j0; j < j1; ++j) {
+                const int64_t i = hc.cell_perm[j];
+                const int64_t g = hc.cell_off + j;
+                const int nf = mv.mesh_connectivity[cidx(n, i, 2)];
+                int nb[4] = {kAbsent, kAbsent, kAbsent, kAbsent};
+                int d1[4] = {0, 0, 0, 0}, u1[4] = {0, 0, 0, 0}, d2[4] = {0, 0, 0, 0}, u2[4] = {0, 0, 0, 0};
+                double per = 0.0;
+                int2 edge[4];
+                for (int k = 0; k < nf; ++k) {
+                    int32_t st = mv.cell_stiffness[cidx(n, i, k)];
+                    if (st >= 1) {
+                        nb[k] = (int32_t)(hc.cell_off + hc.cell_inv[st - 1]);
+                        d1[k] = node_g(mv.node2cellL2down[cidx(n, i, 2 * k)]);
+                        u1[k] = node_g(mv.node2cellL2up[cidx(n, i, 2 * k)]);
+                        if (nf == 4) {
+                            d2[k] = node_g(mv.node2cellL2down[cidx(n, i, 2 * k + 1)]);
+                            u2[k] = node_g(mv.node2cellL2up[cidx(n, i, 2 * k + 1)]);
+                        }
+                    } else {
+                        int slot = 0;
+                        for (int b = 0; b < hc.params.n_bc; ++b) if (hc.params.bc[b].tag == st) { slot = b; break; }
+                        nb[k] = -(slot + 1);
                     }
-                } else {
-                    int slot = 0;
-                    for (int b = 0; b < hc.params.n_bc; ++b) if (hc.params.bc[b].tag == st) { slot = b; break; }
-                    nb[k] = -(slot + 1);
+                    const size_t o = (size_t)k * Nc + g;
+                    gnx[o] = mv.cell_edges_Nx[cidx(n, i, k)];
+                    gny[o] = mv.cell_edges_Ny[cidx(n, i, k)];
+                    glen[o] = mv.cell_edges_length[cidx(n, i, k)];
+                    edge[k] = make_int2(node_g(mv.cells2nodes[cidx(n, i, 2 * k)]), node_g(mv.cells2nodes[cidx(n, i, 2 * k + 1)]));
+                    c2n[o] = edge[k];
+                    per += mv.cell_edges_length[cidx(n, i, k)];
                 }
-                const size_t o = (size_t)k * Nc + g;
-                gnx[o] = mv.cell_edges_Nx[cidx(n, i, k)];
-                gny[o] = mv.cell_edges_Ny[cidx(n, i, k)];
-                glen[o] = mv.cell_edges_length[cidx(n, i, k)];
-                c2n[o] = make_int2(node_g(mv.cells2nodes[cidx(n, i, 2 * k)]), node_g(mv.cells2nodes[cidx(n, i, 2 * k + 1)]));
-                per += mv.cell_edges_length[cidx(n, i, k)];
-            }
-            nbr[g] = make_int4(nb[0], nb[1], nb[2], nb[3]);
-            dn[g] = make_int4(d1[0], d1[1], d1[2], d1[3]);
-            up[g] = make_int4(u1[0], u1[1], u1[2], u1[3]);
-            if (h->quads) { dn2[g] = make_int4(d2[0], d2[1], d2[2], d2[3]); up2[g] = make_int4(u2[0], u2[1], u2[2], u2[3]); }
-            const double A = mv.cell_areas[i];
-            area[g] = A;
-            rarea[g] = 1.0 / A;
-            hx[g] = mv.HX[i];
-            charlen[g] = 2.0 * A / per;
-            if (h->tgv) mid[g] = make_double2(mv.cell_mid_points[cidx(n, i, 0)], mv.cell_mid_points[cidx(n, i, 1)]);
-        }
-        for (int64_t j = 0; j < nn; ++j) {
-            const int64_t J = hc.node_perm[j];
-            const int64_t gn = hc.node_off + j;
-            int slot = 0;
-            for (int q = 0; q < mv.n_neib_cells; ++q) {
-                int32_t cc = mv.cell_clusters[cidx(nn, J, q)];
-                if (cc != 0) {
-                    cl[(size_t)slot * Nn + gn] = (int32_t)(hc.cell_off + hc.cell_inv[cc - 1]);
-                    if (!unit) wt[(size_t)slot * Nn + gn] = mv.node_stencils[cidx(nn, J, q)];
-                    ++slot;
+                if (h->visc) {
+                    // node k is the one that edges k - 1 and k share
+                    int v[4] = {0, 0, 0, 0};
+                    for (int k = 0; k < nf; ++k) {
+                        const int2 p = edge[k ? k - 1 : nf - 1], q = edge[k];
+                        v[k] = (q.x == p.x || q.x == p.y) ? q.x : q.y;
+                    }
+                    bool walk = true;
+                    for (int k = 0; k < nf; ++k) {
+                        const int e0 = v[k], e1 = v[k + 1 < nf ? k + 1 : 0];
+                        walk &= (edge[k].x == e0 && edge[k].y == e1) || (edge[k].x == e1 && edge[k].y == e0);
+                    }
+                    if (!walk) closed = false;
+                    cn[g] = make_int4(v[0], v[1], v[2], v[3]);
                 }
+                nbr[g] = make_int4(nb[0], nb[1], nb[2], nb[3]);
+                dn[g] = make_int4(d1[0], d1[1], d1[2], d1[3]);
+                up[g] = make_int4(u1[0], u1[1], u1[2], u1[3]);
+                if (h->quads) { dn2[g] = make_int4(d2[0], d2[1], d2[2], d2[3]); up2[g] = make_int4(u2[0], u2[1], u2[2], u2[3]); }
+                const double A = mv.cell_areas[i];
+                area[g] = A;
+                rarea[g] = 1.0 / A;
+                hx[g] = mv.HX[i];
+                charlen[g] = 2.0 * A / per;
+                if (h->tgv) mid[g] = make_double2(mv.cell_mid_points[cidx(n, i, 0)], mv.cell_mid_points[cidx(n, i, 1)]);
             }
-            if (h->tgv) { xnode[gn] = mv.x_nodes[J]; ynode[gn] = mv.y_nodes[J]; }
-        }
+        });
+        parallel_ranges(nn, [&](int64_t j0, int64_t j1) {
+            for (int64_t j = j0; j < j1; ++j) {
+                const int64_t J = hc.node_perm[j];
+                const int64_t gn = hc.node_off + j;
+                int slot = 0;
+                for (int q = 0; q < mv.n_neib_cells; ++q) {
+                    int32_t cc = mv.cell_clusters[cidx(nn, J, q)];
+                    if (cc != 0) {
+                        cl[(size_t)slot * Nn + gn] = (int32_t)(hc.cell_off + hc.cell_inv[cc - 1]);
+                        if (!unit) wt[(size_t)slot * Nn + gn] = mv.node_stencils[cidx(nn, J, q)];
+                        ++slot;
+                    }
+                }
+                if (h->tgv) { xnode[gn] = mv.x_nodes[J]; ynode[gn] = mv.y_nodes[J]; }
+            }
+        });
         DevCase d = make_devcase(hc.params, maxEdge);
         d.cell_begin = hc.cell_off;
         d.cell_end = hc.cell_off + hc.nc_pad;
@@ -691,37 +762,9 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
         for (int64_t j = hc.node_off; j < node_end; ++j) node_case[j] = c;
         h->hcases[c] = d;
     }
+    if (!closed) cn.clear();
     h->tile_case_h = tile_case;
     h->ngroups = ngroups;
-
-    // each cell's nodes in edge order, if the edges of every cell are a
-    // closed walk in face order (as the reference's meshes list them): the
-    // gradient passes then gather a node once instead of once per edge.  An
-    // edge's two nodes enter symmetrically, so they may be listed either way.
-    std::vector<int4> cn;
-    if (h->visc) {
-        cn.assign(Nc, make_int4(0, 0, 0, 0));
-        bool closed = true;
-        for (int c = 0; c < n_cases && closed; ++c) {
-            const HostCase &hc = h->cases[c];
-            for (int64_t g = hc.cell_off; g < hc.cell_off + hc.nc && closed; ++g) {
-                const int nf = nbr[g].w != kAbsent ? 4 : 3;
-                int n[4] = {0, 0, 0, 0};
-                for (int k = 0; k < nf; ++k) {
-                    // node k is the one that edges k - 1 and k share
-                    const int2 p = c2n[(size_t)((k + nf - 1) % nf) * Nc + g], q = c2n[(size_t)k * Nc + g];
-                    n[k] = (q.x == p.x || q.x == p.y) ? q.x : q.y;
-                }
-                for (int k = 0; k < nf; ++k) {
-                    const int2 q = c2n[(size_t)k * Nc + g];
-                    const int a = n[k], b = n[(k + 1) % nf];
-                    closed &= (q.x == a && q.y == b) || (q.x == b && q.y == a);
-                }
-                cn[g] = make_int4(n[0], n[1], n[2], n[3]);
-            }
-        }
-        if (!closed) cn.clear();
-    }
 
     // face list for the face-loop variants: each interior face once (from its
     // lower-indexed cell), boundary faces once; greedy edge colouring so that
