@@ -835,8 +835,8 @@ __global__ void __launch_bounds__(256, MINB) k_cell_step_tf(const DevMesh m, con
             if (QUAD && tf.quad) q2 = m.tf_q[f];
             if (rec.x >= 0) {
                 face_nodes<QUAD>(s.nodeP, rec.z, rec.w, q2.x, q2.y, QUAD && tf.quad, up, down);
-                const int64_t lr = (int64_t)rec.x - base;
-                if (lr >= 0 && lr < B) {
+                const unsigned lr = (unsigned)rec.x - (unsigned)base;  // (cell indices fit 31 bits)
+                if (lr < (unsigned)B) {
                     r = s_prim[lr];
                     ehR = s_eh[lr];
                 } else {
@@ -844,7 +844,9 @@ __global__ void __launch_bounds__(256, MINB) k_cell_step_tf(const DevMesh m, con
                     ehR = m.eh[rec.x];
                 }
             }
-            const int64_t og = (int64_t)tf.ka * m.Nc + base + tf.la;
+            // (32-bit plane offsets: 4 planes of the cells that fit the device's
+            // memory stay under 2^32 elements)
+            const unsigned og = (unsigned)tf.ka * (unsigned)m.Nc + (unsigned)base + (unsigned)tf.la;
             double fv[4];
             face_flux_at<FLUX, QUAD>(m, P, s_face, pin, s.nodeP, base + tf.la, tf.ka, rec.x, rec.z, rec.w, q2.x, q2.y,
                                      QUAD && tf.quad, uL, r, up, down, eh_own, ehR, m.len[og], m.nx[og], m.ny[og],
@@ -869,7 +871,7 @@ __global__ void __launch_bounds__(256, MINB) k_cell_step_tf(const DevMesh m, con
         double diff[4] = {0.0, 0.0, 0.0, 0.0};
         if (VISC && live) {
             auto geo = [&](int k, double &nx, double &ny, double &side) {
-                const int64_t o = (int64_t)k * m.Nc + g;
+                const unsigned o = (unsigned)k * (unsigned)m.Nc + (unsigned)g;
                 side = m.len[o];
                 nx = m.nx[o];
                 ny = m.ny[o];
