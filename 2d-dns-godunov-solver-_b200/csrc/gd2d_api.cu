@@ -1116,14 +1116,6 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
     return GD2D_OK;
 }
 
-// Stream-ordered copies on the handle's stream (the handle's stream does not
-// synchronise with the legacy default stream).
-static int copy_sync(gd2d_handle *h, void *dst, const void *src, size_t bytes, cudaMemcpyKind kind) {
-    CUDA_TRY(h, cudaMemcpyAsync(dst, src, bytes, kind, h->stream));
-    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-    return GD2D_OK;
-}
-
 // Transfers between a caller's host columns and the device stage go
 // through the page-locked host stage in slices of 2 MB, handed out in order
 // to the handle's worker threads (StagePool, at most 8 threads with the
@@ -1253,13 +1245,15 @@ static int drop_graph(gd2d_handle *h) {
 // Where the primitives of a case are written before its initialisation:
 // FP64, the current primitive buffer; mixed, U, which the init kernel turns
 // into conservatives while writing the FP32 primitives.
-static int case_prims_dst(gd2d_handle *h, int32_t icase, double4 **dst) {
-    const HostCase &hc = h->cases[icase];
-    int par = 0;
-    int rc = copy_sync(h, &par, h->s.parity, sizeof(int), cudaMemcpyDeviceToHost);
-    if (rc) return rc;
-    *dst = h->mixed ? h->s.U + hc.cell_off : h->s.prim + (int64_t)par * h->m.Nc + hc.cell_off;
-    return GD2D_OK;
+struct PrimsDst {
+    double4 *dst;
+    const int32_t *parity;
+    int64_t buffer;
+};
+static PrimsDst case_prims_dst(const gd2d_handle *h, int32_t icase) {
+    const int64_t off = h->cases[icase].cell_off;
+    if (h->mixed) return {h->s.U + off, nullptr, 0};
+    return {h->s.prim + off, h->s.parity, h->m.Nc};
 }
 
 // The case's primitives, already in place (case_prims_dst), become its
@@ -1279,14 +1273,16 @@ static int init_case(gd2d_handle *h, int32_t icase, double t0, bool nodes_from_c
     if (h->mixed) {
         CUDA_TRY(h, launch_init_state_mixed(h->m, h->s, d.tile_begin, d.tile_end, h->lc, h->stream));
         if (exact_cons)
-            CUDA_TRY(h, launch_cols_to_dev(exact_cons, h->d_perm + hc.cell_off, hc.nc, h->s.U + hc.cell_off, h->stream));
+            CUDA_TRY(h, launch_cols_to_dev(exact_cons, h->d_perm + hc.cell_off, hc.nc, h->s.U + hc.cell_off, nullptr, 0,
+                                           h->stream));
         CUDA_TRY(h, launch_node_avg_mixed(h->m, h->s, h->visc, false, !nodes_from_cells, hc.node_off,
                                           hc.node_off + hc.nn, d.group_begin, d.group_end, true, h->lc,
                                           h->stream));
     } else {
         CUDA_TRY(h, launch_init_state_f64(h->m, h->s, d.tile_begin, d.tile_end, h->lc, h->stream));
         if (exact_cons)
-            CUDA_TRY(h, launch_cols_to_dev(exact_cons, h->d_perm + hc.cell_off, hc.nc, h->s.U + hc.cell_off, h->stream));
+            CUDA_TRY(h, launch_cols_to_dev(exact_cons, h->d_perm + hc.cell_off, hc.nc, h->s.U + hc.cell_off, nullptr, 0,
+                                           h->stream));
         CUDA_TRY(h, launch_node_avg_f64(h->m, h->s, h->visc, false, !nodes_from_cells, hc.node_off,
                                         hc.node_off + hc.nn, d.group_begin, d.group_end, true, h->lc,
                                         h->stream));
@@ -1307,12 +1303,11 @@ int gd2d_set_state(gd2d_handle *h, int32_t icase, const double *density, const d
     if (!density || !ux || !uy || !pressure) return fail(h, GD2D_ERR_ARG, "NULL field pointer");
     cudaSetDevice(h->device);
     const HostCase &hc = h->cases[icase];
-    double4 *dst = nullptr;
-    if ((rc = case_prims_dst(h, icase, &dst))) return rc;
+    const PrimsDst to = case_prims_dst(h, icase);
     const int64_t n = hc.nc;
     const double *cols[4] = {density, ux, uy, pressure};
     if ((rc = staged_upload(h, cols, n))) return rc;
-    CUDA_TRY(h, launch_cols_to_dev(h->d_stage, h->d_perm + hc.cell_off, n, dst, h->stream));
+    CUDA_TRY(h, launch_cols_to_dev(h->d_stage, h->d_perm + hc.cell_off, n, to.dst, to.parity, to.buffer, h->stream));
     return init_case(h, icase, hc.start_time, hc.params.init_nodes != 0);
 }
 
@@ -1322,12 +1317,12 @@ int gd2d_set_conservative(gd2d_handle *h, int32_t icase, const double *ucons, do
     if (!ucons) return fail(h, GD2D_ERR_ARG, "NULL ucons");
     cudaSetDevice(h->device);
     const HostCase &hc = h->cases[icase];
-    double4 *dst = nullptr;
-    if ((rc = case_prims_dst(h, icase, &dst))) return rc;
+    const PrimsDst to = case_prims_dst(h, icase);
     const int64_t n = hc.nc;
     const double *cols[4] = {ucons, ucons + n, ucons + 2 * n, ucons + 3 * n};
     if ((rc = staged_upload(h, cols, n))) return rc;
-    CUDA_TRY(h, launch_cons_to_prims(h->d_stage, h->d_perm + hc.cell_off, n, hc.params.Gamma, dst, h->stream));
+    CUDA_TRY(h, launch_cons_to_prims(h->d_stage, h->d_perm + hc.cell_off, n, hc.params.Gamma, to.dst, to.parity,
+                                     to.buffer, h->stream));
     return init_case(h, icase, flow_time, rebuild_nodes != 0, h->d_stage);
 }
 
@@ -1556,12 +1551,14 @@ int gd2d_get_history(gd2d_handle *h, int32_t icase, gd2d_stats *out, int32_t cap
 }
 
 // One device-order field of a case, reordered on the device into the
-// staging columns and copied to a column-major host matrix.
+// staging columns and copied to a column-major host matrix; `current` for the
+// current buffer of the primitives.
 static int download_rows(gd2d_handle *h, const double4 *src, const float4 *srcf, const int32_t *inv, int64_t n,
-                         double *dst) {
+                         double *dst, bool current = false) {
     if (!dst) return GD2D_OK;
-    CUDA_TRY(h, srcf ? launch_dev_to_cols_f(srcf, inv, n, h->d_stage, h->stream)
-                     : launch_dev_to_cols(src, inv, n, h->d_stage, h->stream));
+    const int32_t *parity = current ? h->s.parity : nullptr;
+    CUDA_TRY(h, srcf ? launch_dev_to_cols_f(srcf, inv, n, h->d_stage, parity, h->m.Nc, h->stream)
+                     : launch_dev_to_cols(src, inv, n, h->d_stage, parity, h->m.Nc, h->stream));
     return staged_download(h, dst, n);
 }
 
@@ -1570,18 +1567,13 @@ int gd2d_get_state(gd2d_handle *h, int32_t icase, double *ucons, double *prims, 
     if (rc) return rc;
     cudaSetDevice(h->device);
     HostCase &hc = h->cases[icase];
-    int par = 0;
-    rc = copy_sync(h, &par, h->s.parity, sizeof(int), cudaMemcpyDeviceToHost);
-    if (rc) return rc;
     const int32_t *inv = h->d_inv + hc.ref_off, *ninv = h->d_ninv + hc.nref_off;
     if ((rc = download_rows(h, h->s.U + hc.cell_off, nullptr, inv, hc.nc, ucons))) return rc;
     if (h->mixed) {
-        if ((rc = download_rows(h, nullptr, h->s.primf + (int64_t)par * h->m.Nc + hc.cell_off, inv, hc.nc, prims)))
-            return rc;
+        if ((rc = download_rows(h, nullptr, h->s.primf + hc.cell_off, inv, hc.nc, prims, true))) return rc;
         if ((rc = download_rows(h, nullptr, h->s.nodePf + hc.node_off, ninv, hc.nn, node_prims))) return rc;
     } else {
-        if ((rc = download_rows(h, h->s.prim + (int64_t)par * h->m.Nc + hc.cell_off, nullptr, inv, hc.nc, prims)))
-            return rc;
+        if ((rc = download_rows(h, h->s.prim + hc.cell_off, nullptr, inv, hc.nc, prims, true))) return rc;
         if ((rc = download_rows(h, h->s.nodeP + hc.node_off, nullptr, ninv, hc.nn, node_prims))) return rc;
     }
     return GD2D_OK;

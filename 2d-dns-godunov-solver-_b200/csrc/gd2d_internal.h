@@ -221,12 +221,16 @@ cudaError_t launch_cell_step_tf_f64(const DevMesh &m, const DevState &s, int flu
                                     const LaunchCfg &lc, cudaStream_t st);
 // Reordering between the reference's column-major rows and device order
 // (cols: [n x 4] column-major; perm[j] = reference row of device record j;
-// inv[i] = device record of reference row i).
-cudaError_t launch_cols_to_dev(const double *cols, const int32_t *perm, int64_t n, double4 *dst, cudaStream_t st);
+// inv[i] = device record of reference row i).  With `parity` the device field
+// is the buffer of that parity, `buffer` records after the one given.
+cudaError_t launch_cols_to_dev(const double *cols, const int32_t *perm, int64_t n, double4 *dst, const int32_t *parity,
+                               int64_t buffer, cudaStream_t st);
 cudaError_t launch_cons_to_prims(const double *cols, const int32_t *perm, int64_t n, double gamma, double4 *dst,
-                                 cudaStream_t st);
-cudaError_t launch_dev_to_cols(const double4 *src, const int32_t *inv, int64_t n, double *cols, cudaStream_t st);
-cudaError_t launch_dev_to_cols_f(const float4 *src, const int32_t *inv, int64_t n, double *cols, cudaStream_t st);
+                                 const int32_t *parity, int64_t buffer, cudaStream_t st);
+cudaError_t launch_dev_to_cols(const double4 *src, const int32_t *inv, int64_t n, double *cols, const int32_t *parity,
+                               int64_t buffer, cudaStream_t st);
+cudaError_t launch_dev_to_cols_f(const float4 *src, const int32_t *inv, int64_t n, double *cols,
+                                 const int32_t *parity, int64_t buffer, cudaStream_t st);
 // Node pass over nodes [n0, n1).  Its first blocks also complete the step
 // reduction of the tile records of groups [g0, g1) that the cell kernel (or
 // the state initialisation, red_init) wrote: the last group of each case

@@ -147,6 +147,10 @@ cudaError_t launch_diff_only_f64(const DevMesh &m, const DevState &s, double4 *d
 // matrices (or four columns) indexed by the reference's cell / node ids.
 // These kernels do the reordering on the device, so the host only copies
 // contiguous blocks (a permutation on the host is a cache miss per value).
+// A field that is double-buffered by step parity is given by its first
+// buffer, the parity flag and the distance of the second: read here, the
+// flag costs a call no copy to the host and no wait (15 us of the 80-120 us
+// that setting or reading a small case takes).
 
 namespace gd2d {
 
@@ -164,7 +168,9 @@ int reorder_grid(int64_t n) {
 __global__ void __launch_bounds__(256) k_cols_to_dev(const double *__restrict__ a, const double *__restrict__ b,
                                                      const double *__restrict__ c, const double *__restrict__ d,
                                                      const int32_t *__restrict__ perm, int64_t n,
-                                                     double4 *__restrict__ dst) {
+                                                     double4 *__restrict__ dst, const int32_t *parity,
+                                                     int64_t buffer) {
+    if (parity) dst += *parity * buffer;
     for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
         const int64_t i = perm[j];
         dst[j] = make_double4(a[i], b[i], c[i], d[i]);
@@ -177,7 +183,9 @@ __global__ void __launch_bounds__(256) k_cols_to_dev(const double *__restrict__ 
 // replaces.
 __global__ void __launch_bounds__(256) k_cons_to_prims(const double *__restrict__ u, int64_t n,
                                                        const int32_t *__restrict__ perm, double G,
-                                                       double4 *__restrict__ dst) {
+                                                       double4 *__restrict__ dst, const int32_t *parity,
+                                                       int64_t buffer) {
+    if (parity) dst += *parity * buffer;
     for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
         const int64_t i = perm[j];
         const double U1 = u[i], U2 = u[i + n], U3 = u[i + 2 * n], U4 = u[i + 3 * n];
@@ -189,7 +197,9 @@ __global__ void __launch_bounds__(256) k_cons_to_prims(const double *__restrict_
 // reference-order columns (FP32 records widened exactly).
 template <class T4>
 __global__ void __launch_bounds__(256) k_dev_to_cols(const T4 *__restrict__ src, const int32_t *__restrict__ inv,
-                                                     int64_t n, double *__restrict__ dst) {
+                                                     int64_t n, double *__restrict__ dst, const int32_t *parity,
+                                                     int64_t buffer) {
+    if (parity) src += *parity * buffer;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const T4 r = src[inv[i]];
         dst[i] = (double)r.x;
@@ -201,24 +211,28 @@ __global__ void __launch_bounds__(256) k_dev_to_cols(const T4 *__restrict__ src,
 
 }  // namespace
 
-cudaError_t launch_cols_to_dev(const double *cols, const int32_t *perm, int64_t n, double4 *dst, cudaStream_t st) {
-    k_cols_to_dev<<<reorder_grid(n), 256, 0, st>>>(cols, cols + n, cols + 2 * n, cols + 3 * n, perm, n, dst);
+cudaError_t launch_cols_to_dev(const double *cols, const int32_t *perm, int64_t n, double4 *dst, const int32_t *parity,
+                               int64_t buffer, cudaStream_t st) {
+    k_cols_to_dev<<<reorder_grid(n), 256, 0, st>>>(cols, cols + n, cols + 2 * n, cols + 3 * n, perm, n, dst, parity,
+                                                   buffer);
     return cudaGetLastError();
 }
 
 cudaError_t launch_cons_to_prims(const double *cols, const int32_t *perm, int64_t n, double gamma, double4 *dst,
-                                 cudaStream_t st) {
-    k_cons_to_prims<<<reorder_grid(n), 256, 0, st>>>(cols, n, perm, gamma, dst);
+                                 const int32_t *parity, int64_t buffer, cudaStream_t st) {
+    k_cons_to_prims<<<reorder_grid(n), 256, 0, st>>>(cols, n, perm, gamma, dst, parity, buffer);
     return cudaGetLastError();
 }
 
-cudaError_t launch_dev_to_cols(const double4 *src, const int32_t *inv, int64_t n, double *cols, cudaStream_t st) {
-    k_dev_to_cols<double4><<<reorder_grid(n), 256, 0, st>>>(src, inv, n, cols);
+cudaError_t launch_dev_to_cols(const double4 *src, const int32_t *inv, int64_t n, double *cols, const int32_t *parity,
+                               int64_t buffer, cudaStream_t st) {
+    k_dev_to_cols<double4><<<reorder_grid(n), 256, 0, st>>>(src, inv, n, cols, parity, buffer);
     return cudaGetLastError();
 }
 
-cudaError_t launch_dev_to_cols_f(const float4 *src, const int32_t *inv, int64_t n, double *cols, cudaStream_t st) {
-    k_dev_to_cols<float4><<<reorder_grid(n), 256, 0, st>>>(src, inv, n, cols);
+cudaError_t launch_dev_to_cols_f(const float4 *src, const int32_t *inv, int64_t n, double *cols,
+                                 const int32_t *parity, int64_t buffer, cudaStream_t st) {
+    k_dev_to_cols<float4><<<reorder_grid(n), 256, 0, st>>>(src, inv, n, cols, parity, buffer);
     return cudaGetLastError();
 }
 
