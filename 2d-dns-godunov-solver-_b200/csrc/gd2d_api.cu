@@ -213,6 +213,7 @@ void parallel_ranges(int64_t n, const Fn &fn) {
     const int64_t nt = std::min<int64_t>({8, (int64_t)std::max(1u, std::thread::hardware_concurrency()), n / least});
     if (nt <= 1) return fn((int64_t)0, n);
     std::vector<std::thread> th;
+    th.reserve((size_t)nt);  // (no allocation once a thread runs)
     int64_t begin = 0;
     try {
         for (int64_t t = 0; t + 1 < nt; ++t) {
@@ -220,7 +221,7 @@ void parallel_ranges(int64_t n, const Fn &fn) {
             th.emplace_back([&fn, begin, end] { fn(begin, end); });
             begin = end;
         }
-    } catch (const std::system_error &) {
+    } catch (const std::exception &) {  // no thread to be had: the caller does the rest
     }
     fn(begin, n);
     for (auto &t : th) t.join();

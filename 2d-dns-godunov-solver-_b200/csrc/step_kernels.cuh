@@ -3,9 +3,11 @@
 // One step = [viscous: grad1 cell pass, grad1 node pass] -> fused cell
 // kernel -> node kernel.  The fused cell kernel does, per cell,
 // calcOneStageMUSCLcpuFast (calcOneStageMUSCLcpuFast.jl:3-107) followed by
-// updateVariablesSA (evaluate2d.jl:52-110) and the step's reductions; the
-// last tile of each case finalizes that case's statistics and next time step
-// (no device-wide barrier, no spin: a per-case ticket counter elects it).
+// updateVariablesSA (evaluate2d.jl:52-110) and writes its tile's reduction
+// record; the first blocks of the node kernel fold a case's records and
+// finalize its statistics and next time step (no device-wide barrier, no
+// spin: a case of one tile group is folded by one block, in a larger one a
+// counter elects the last warp).
 #pragma once
 
 #include <cuda_runtime.h>
