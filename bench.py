@@ -48,10 +48,10 @@ CELL_ALG_BYTES = {("f64", False): 180, ("f64", True): 212, ("mixed", False): 140
 
 # DRAM bytes per cell of one cell-kernel launch on the viscous cylinder,
 # measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum of one
-# launch; FP64 cell-centred on 1025^2 nodes, the others on 513^2 nodes, the
-# traffic growing in proportion to the cells); None where not captured.
-CELL_KERNEL_TRAFFIC = {("f64", "cell"): 337.0, ("f64", "tile"): 282.0, ("mixed", "cell"): 233.0,
-                       ("mixed", "tile"): 149.0}
+# launch on 513^2 nodes, the traffic growing in proportion to the cells);
+# None where not captured.
+CELL_KERNEL_TRAFFIC = {("f64", "cell"): 322.0, ("f64", "tile"): 284.0, ("mixed", "cell"): 227.0,
+                       ("mixed", "tile"): 180.0}
 
 
 def load_peaks():
