@@ -5,7 +5,8 @@
 // straddles two cases):
 //   per cell  : int4 nbr (neighbour cell or -(bc_slot+1), kAbsent for no face),
 //               int4 dn/up (down/up node per face; quads: dn2/up2 second node),
-//               int2 c2n[k] (edge node pair, viscous and TGV only),
+//               int4 cn (the nodes in face order, viscous),
+//               int2 c2n[k] (edge node pairs: TGV, and viscous meshes without cn),
 //               geometry planes nx[k], ny[k], len[k] (k < faces), rarea, area,
 //               hx, charlen, mid (x,y);
 //   state     : double4 U (rho, rho u, rho v, E) updated in place,
