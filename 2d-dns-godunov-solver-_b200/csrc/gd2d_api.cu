@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "../../include/godunov2d.h"
+#include "exact_case.h"
 #include "gd2d_internal.h"
 
 using namespace gd2d;
@@ -414,25 +415,6 @@ DevCase make_devcase(const gd2d_params &p, double maxEdge) {
     return d;
 }
 
-// Whether a case's constants and cell geometry are in the range for which the
-// straight-line quotients of face_exact.cuh round correctly (any case in
-// physical units is); if not, its cells are evaluated by the plain formulas.
-bool exact_rows_case(const DevCase &d, const gd2d_mesh_view &mv) {
-    auto in = [](double x, double lo, double hi) { return x >= lo && x <= hi; };  // false for NaN
-    // divisors with an all-ones significand are the method's exception
-    auto divisor = [&](double x) {
-        uint64_t b;
-        std::memcpy(&b, &x, sizeof b);
-        return in(x, 1e-20, 1e20) && (b & 0xffffffffu) != 0xffffffffu;
-    };
-    if (!divisor(d.face.gm1) || !divisor(d.R) || !in(d.gamma, 1.01, 100.0)) return false;
-    if (d.visc_model == VISC_SUTHERLAND && !divisor(d.suth_ref)) return false;
-    if (!in(d.venkat_K, 0.0, 1e6) || !in(d.ksi, 0.0, 1e20)) return false;
-    for (int64_t i = 0; i < mv.n_cells; ++i)
-        if (!divisor(mv.cell_areas[i]) || !divisor(mv.HX[i])) return false;
-    return true;
-}
-
 template <class T>
 cudaError_t upload(T *dst, const std::vector<T> &src) {
     if (src.empty()) return cudaSuccess;
@@ -757,7 +739,7 @@ int gd2d_setup(gd2d_handle **out, int32_t n_cases, const gd2d_mesh_view *meshes,
         d.group_begin = ngroups;
         ngroups += (d.tile_end - d.tile_begin + kGroupTiles - 1) / kGroupTiles;
         d.group_end = ngroups;
-        d.face.exact_rows = exact_rows_case(d, mv) ? 1 : 0;
+        d.face.exact_rows = exact_rows_case(d, mv.n_cells, mv.cell_areas, mv.HX) ? 1 : 0;
         for (int64_t t = d.tile_begin; t < d.tile_end; ++t) tile_case[t] = c;
         const int64_t node_end = (c + 1 < n_cases) ? h->cases[c + 1].node_off : Nn;
         for (int64_t j = hc.node_off; j < node_end; ++j) node_case[j] = c;
