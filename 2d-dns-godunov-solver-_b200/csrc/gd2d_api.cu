@@ -1216,7 +1216,10 @@ static int ensure_case(gd2d_handle *h, int32_t icase) {
     return GD2D_OK;
 }
 
+// Forgets what was captured, and timed, for the launch shape in use.
 static int drop_graph(gd2d_handle *h) {
+    h->last_cell_ms = 0.0;
+    h->single_calls = 0;
     if (h->graph) { cudaGraphExecDestroy(h->graph); h->graph = nullptr; }
     if (h->graph1) { cudaGraphExecDestroy(h->graph1); h->graph1 = nullptr; }
     if (h->graph1_timed) { cudaGraphExecDestroy(h->graph1_timed); h->graph1_timed = nullptr; }
@@ -1519,7 +1522,7 @@ int gd2d_propagate(gd2d_handle *h, int32_t nsteps, gd2d_stats *stats_out) {
                              (long long)(step0[0] + chunk));
     }
     h->last_total_ms = total_ms;
-    if (cell_samples) h->last_cell_ms = cell_ms / cell_samples;
+    if (cell_samples || nsteps == 0) h->last_cell_ms = cell_samples ? cell_ms / cell_samples : 0.0;
     h->last_launches = launches;
     return GD2D_OK;
 }

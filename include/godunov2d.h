@@ -231,7 +231,9 @@ int gd2d_autotune(gd2d_handle *h, int32_t steps_per_trial, gd2d_launch *chosen);
  * handle's stream): total ms and ms of the fused cell kernel.  The cell
  * kernel is timed on one step of a call (the last one of the call's last
  * step graph, or of the call); of calls of one step, the first and every
- * 32nd after it are timed and the others report the last one timed. */
+ * 32nd after it are timed and the others report the last one timed.  A call
+ * of no steps reports zeros, and gd2d_autotune discards the time of the
+ * shape that it replaces (0 until the next call that is timed). */
 int gd2d_last_timing(gd2d_handle *h, double *total_ms, double *cell_kernel_ms, int64_t *launches);
 
 int gd2d_destroy(gd2d_handle *h);
