@@ -146,9 +146,8 @@ struct gd2d_handle {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     cudaGraphExec_t graph = nullptr;
-    cudaGraphExec_t graph1 = nullptr;        // one step, for a propagate call's single leftover step
-    cudaGraphExec_t graph1_timed = nullptr;  // the same with its cell kernel timed
-    int64_t single_calls = 0;                // one-step propagate calls so far
+    cudaGraphExec_t graph1 = nullptr;  // one step, for a propagate call's single leftover step
+    int64_t single_calls = 0;          // one-step propagate calls so far
     int graph_steps = 0;
     bool state_ready = false;
     std::vector<std::vector<gd2d_stats>> history;
@@ -1222,7 +1221,6 @@ static int drop_graph(gd2d_handle *h) {
     h->single_calls = 0;
     if (h->graph) { cudaGraphExecDestroy(h->graph); h->graph = nullptr; }
     if (h->graph1) { cudaGraphExecDestroy(h->graph1); h->graph1 = nullptr; }
-    if (h->graph1_timed) { cudaGraphExecDestroy(h->graph1_timed); h->graph1_timed = nullptr; }
     for (cudaEvent_t e : h->ev) cudaEventDestroy(e);
     h->ev.clear();
     return GD2D_OK;
@@ -1412,13 +1410,11 @@ static int capture_graph(gd2d_handle *h, int steps, bool timing) {
     return end_capture(h, first, &h->graph, "step graph");
 }
 
-// A one-step graph, for a call's single leftover step; with `timing` its cell
-// kernel is bracketed by the eager event pair.
-static int capture_step_graph(gd2d_handle *h, bool timing, cudaGraphExec_t *out) {
+// A one-step graph, for a call's single leftover step.
+static int capture_step_graph(gd2d_handle *h) {
     CUDA_TRY(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    const cudaError_t first = launch_step_kernels(h, timing ? h->ev_eager[0] : nullptr,
-                                                  timing ? h->ev_eager[1] : nullptr, true);
-    return end_capture(h, first, out, "one-step graph");
+    const cudaError_t first = launch_step_kernels(h, nullptr, nullptr, true);
+    return end_capture(h, first, &h->graph1, "one-step graph");
 }
 
 int gd2d_propagate(gd2d_handle *h, int32_t nsteps, gd2d_stats *stats_out) {
@@ -1451,12 +1447,14 @@ int gd2d_propagate(gd2d_handle *h, int32_t nsteps, gd2d_stats *stats_out) {
         // graph); a single one, the step-by-step caller's case, is a graph
         // of its own, which costs the host less than its launches.  The
         // event records around its cell kernel would cost it a fifth, so a
-        // caller stepping one at a time has one step in 32 timed.
-        const bool single = G > 1 && chunk % G == 1;
-        const bool time_single = single && chunk == 1 && h->single_calls++ % 32 == 0;
-        cudaGraphExec_t &g1 = time_single ? h->graph1_timed : h->graph1;
-        if (single && !g1) {
-            int rc = capture_step_graph(h, time_single, &g1);
+        // caller stepping one at a time has one step in 32 timed, launched
+        // kernel by kernel.  As a second graph it cost a handle a second
+        // capture: 281 us for its first two calls (2,048 cells) instead of
+        // 202.
+        const bool timed_single = chunk == 1 && h->single_calls++ % 32 == 0;
+        const bool single = G > 1 && chunk % G == 1 && !timed_single;
+        if (single && !h->graph1) {
+            int rc = capture_step_graph(h);
             if (rc) return rc;
         }
         CUDA_TRY(h, cudaEventRecord(h->ev_total[0], h->stream));
@@ -1473,7 +1471,7 @@ int gd2d_propagate(gd2d_handle *h, int32_t nsteps, gd2d_stats *stats_out) {
         const bool time_eager = !used_graph && !single && k < chunk;
         for (; k < chunk; ++k) {
             if (single) {
-                CUDA_TRY(h, cudaGraphLaunch(g1, h->stream));
+                CUDA_TRY(h, cudaGraphLaunch(h->graph1, h->stream));
             } else {
                 const bool last = time_eager && k == chunk - 1;
                 CUDA_TRY(h, launch_step_kernels(h, last ? h->ev_eager[0] : nullptr, last ? h->ev_eager[1] : nullptr));
@@ -1495,7 +1493,7 @@ int gd2d_propagate(gd2d_handle *h, int32_t nsteps, gd2d_stats *stats_out) {
                 ++cell_samples;
             }
             (void)cudaGetLastError();  // a failed timing query must not surface at the next launch
-        } else if (time_eager || time_single) {
+        } else if (time_eager) {
             float c = 0.f;
             if (cudaEventElapsedTime(&c, h->ev_eager[0], h->ev_eager[1]) == cudaSuccess) {
                 cell_ms += c;
