@@ -27,6 +27,7 @@
 // took 790 us (0.68 TB/s).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <mutex>
@@ -37,17 +38,19 @@
 
 namespace {
 
-constexpr int64_t kNoAllocMaxCells = int64_t(1) << 24;  // 16,777,216 cells
+// The entry point's documented limit, 16,777,216 cells; the scratch does not
+// set it (a record a block, however many cells the block takes).
+constexpr int64_t kNoAllocMaxCells = int64_t(1) << 24;
 constexpr int kNoAllocTile = 256;
-constexpr int64_t kNoAllocMaxTiles = kNoAllocMaxCells / kNoAllocTile;  // 65,536
 constexpr int kRec = 8;  // res[4], vmax, bad, 2 spare
 constexpr int kNoAllocBlocksPerSm = 4;
+constexpr int64_t kNoAllocMaxBlocks = 1024;  // records there is room for (592 blocks on 148 SMs)
 // Records, then 256 bytes holding the ticket counter (first 4 bytes).
-constexpr int64_t kScratchDoubles = kNoAllocMaxTiles * kRec + 32;
+constexpr int64_t kScratchDoubles = kNoAllocMaxBlocks * kRec + 32;
 
 }  // namespace
 
-// 4 MiB + 256 B per GPU: the whole scratch of this entry point.
+// 64 KiB + 256 B per GPU: the whole scratch of this entry point.
 static __device__ __align__(256) double g_noalloc_scratch[kScratchDoubles];
 
 namespace {
@@ -92,7 +95,7 @@ k_update_variables_noalloc(const double *__restrict__ unew, double *__restrict__
                            int64_t n, double G, double *scratch, double *stats_out) {
     __shared__ Red sh[kNoAllocTile / 32];
     __shared__ int s_last;
-    unsigned int *ticket = reinterpret_cast<unsigned int *>(scratch + kNoAllocMaxTiles * kRec);
+    unsigned int *ticket = reinterpret_cast<unsigned int *>(scratch + kNoAllocMaxBlocks * kRec);
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     Red a{0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -198,7 +201,7 @@ extern "C" int gd2d_update_variables_noalloc(const double *d_unew, double *d_uol
     if (n_cells <= 0 || n_cells > kNoAllocMaxCells) {
         char buf[256];
         snprintf(buf, sizeof buf,
-                 "gd2d_update_variables_noalloc: n_cells=%lld outside 1..%lld (fixed scratch of this entry point)",
+                 "gd2d_update_variables_noalloc: n_cells=%lld outside 1..%lld (the limit of this entry point)",
                  (long long)n_cells, (long long)kNoAllocMaxCells);
         return noalloc_fail(GD2D_ERR_ARG, buf);
     }
@@ -233,12 +236,13 @@ extern "C" int gd2d_update_variables_noalloc(const double *d_unew, double *d_uol
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int64_t ntiles = (n_cells + kNoAllocTile - 1) / kNoAllocTile;
     // the ticket counter must start at zero (a previous call may have failed)
-    e = cudaMemsetAsync(scratch + kNoAllocMaxTiles * kRec, 0, 256, st);
+    e = cudaMemsetAsync(scratch + kNoAllocMaxBlocks * kRec, 0, 256, st);
     if (e != cudaSuccess) return noalloc_fail(GD2D_ERR_CUDA, cudaGetErrorString(e));
     int sms = 0;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return noalloc_fail(GD2D_ERR_CUDA, cudaGetErrorString(e));
-    const int64_t blocks = ntiles < (int64_t)sms * kNoAllocBlocksPerSm ? ntiles : (int64_t)sms * kNoAllocBlocksPerSm;
+    const int64_t fit = std::min<int64_t>((int64_t)sms * kNoAllocBlocksPerSm, kNoAllocMaxBlocks);
+    const int64_t blocks = std::min(ntiles, fit);
     k_update_variables_noalloc<<<(unsigned int)blocks, kNoAllocTile, 0, st>>>(d_unew, d_uold, d_prims, n_cells, gamma,
                                                                              scratch, d_stats);
     e = cudaGetLastError();

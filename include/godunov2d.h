@@ -246,8 +246,8 @@ int gd2d_destroy(gd2d_handle *h);
  * d_unew, d_uold, d_prims: [n_cells x 4] column-major device arrays (d_uold is
  * overwritten with d_unew, d_prims receives rho, u, v, p); d_stats: 6 device
  * doubles = sum of (Unew-Uold)^2 per variable, max VMAX, non-finite flag.
- * The only scratch is a fixed 4 MiB array inside the library (one per GPU,
- * held until exit), so n_cells is limited to 16,777,216 (larger: GD2D_ERR_ARG).
+ * n_cells is limited to 16,777,216 (larger: GD2D_ERR_ARG).  The only scratch
+ * is a fixed array of 64 KiB inside the library (one per GPU, held until exit).
  * The first call on a device looks that array up (again after the device's
  * context is recreated, e.g. by cudaDeviceReset) and should come before any
  * stream capture; calls that overlap on the GPU share the array and race.
