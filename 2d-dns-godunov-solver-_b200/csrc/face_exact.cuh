@@ -99,7 +99,7 @@ __device__ __forceinline__ bool ausm_plus_exact(const double *L, const double *R
     const double wL = fabs(vnL) > sL ? fabs(vnL) : sL, wR = fabs(vnR) > sR ? fabs(vnR) : sR;
     const double aL = sL * div_rn(sL, wL), aR = sR * div_rn(sR, wR);
     const double a12 = aR < aL ? aR : aL;
-    Divisors<-700, 210> dr(rhoL);
+    Divisors<-700, 200> dr(rhoL);
     dr.add(rhoR);
     dr.add(wL);
     dr.add(wR);
@@ -160,7 +160,7 @@ __device__ __forceinline__ bool roe_exact(const double *L, const double *R, doub
     // 2 a a is twice a a, and so are their reciprocals one half
     const double LdU1 = div_by(n1, 2.0 * aa, 0.5 * yaa), LdU2 = rho * dum, LdU3 = drho - div_by(dp, aa, yaa);
     const double LdU4 = div_by(n4, 2.0 * aa, 0.5 * yaa);
-    Divisors<-400, 210> d(rhoL);
+    Divisors<-400, 200> d(rhoL);
     d.add(rhoR);
     d.add(w);
     d.add(aa);

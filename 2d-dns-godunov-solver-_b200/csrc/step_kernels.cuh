@@ -250,7 +250,7 @@ __device__ __forceinline__ void fold_warps(const DevMesh &m, const DevState &s, 
 // holds kPartials doubles a warp), folded by the first threads.  With
 // ALIASED, `shares` overlays buffers the block used for the tile, so a
 // barrier retires them first.  Nothing more happens at the tile's end: the
-// next node pass folds the records (fold_field), so no tile waits for a
+// next node pass folds the records (fold_block), so no tile waits for a
 // fence or an atomic.  The last barrier retires `shares`.
 template <bool FIELD_MAJOR, bool ALIASED>
 __device__ __forceinline__ void tile_record(const DevMesh &m, const DevState &s, int64_t tile, const Part &p,
