@@ -544,6 +544,8 @@ __device__ __forceinline__ bool diff_model_exact(const DevCase &P, const double4
     if (P.visc_model == VISC_REFERENCE || !P.face.exact_rows) return false;
     Numerators n(sx[0]);
     n.add(sy[0]);
+    Below<700> big(sx[0]);
+    big.add(sy[0]);
     double lap[3];
 #pragma unroll
     for (int v = 0; v < 3; ++v) {
@@ -551,11 +553,10 @@ __device__ __forceinline__ bool diff_model_exact(const DevCase &P, const double4
         if (v > 0) {
             n.add(sx[v]);
             n.add(sy[v]);
+            big.add(sx[v]);
+            big.add(sy[v]);
         }
     }
-    Finite fin(lap[0]);
-    fin.add(lap[1]);
-    fin.add(lap[2]);
     InRange<-150, 200> r(me.w);
     Divisors<-150, 200> d(me.x);
     const double yrho = rcp_rn(me.x);
@@ -571,13 +572,14 @@ __device__ __forceinline__ bool diff_model_exact(const DevCase &P, const double4
     if (art) {
         // (a divergence too small to be rounded right is far above -a)
         divU = div_by(du, area, rarea) + div_by(dv, area, rarea);
-        fin.add(divU);
+        big.add(du);
+        big.add(dv);
         const double aS2 = div_by(P.gamma * me.w, me.x, yrho);
         r.add(aS2);
         const double root2 = sqrt(2.0);
         a = div_by(div_rn(0.05 * sqrt_rn(aS2), HX), root2, 1.0 / root2);
     }
-    if (!n.ok() || !r.ok() || !d.ok() || !fin.ok()) return false;
+    if (!n.ok() || !r.ok() || !d.ok() || !big.ok()) return false;
     const double mue = mu + (art ? art_viscosity(me.x, HX, divU, a) : 0.0);
     diff[1] = mue * lap[0];
     diff[2] = mue * lap[1];
@@ -1095,28 +1097,24 @@ __global__ void __launch_bounds__(256, GD2D_NODE_MINB) k_grad1_cells(const DevMe
         }
         if (area == 0.0) continue;
         // six quotients over one area (face_exact.cuh's range: the area's is
-        // the case's, a sum too small to be divided right, or one whose
-        // quotient is not finite, takes the plain `/`)
+        // the case's, a sum too small or too large to be divided right takes
+        // the plain `/`)
         const double y = rcp_rn(area);
         double qx[3], qy[3];
         Numerators n(sx[0]);
-        n.add(sy[0]);
+        Below<700> big(sx[0]);
 #pragma unroll
         for (int v = 0; v < 3; ++v) {
             qx[v] = div_by(sx[v], area, y);
             qy[v] = div_by(sy[v], area, y);
             if (v > 0) {
                 n.add(sx[v]);
-                n.add(sy[v]);
+                big.add(sx[v]);
             }
+            n.add(sy[v]);
+            big.add(sy[v]);
         }
-        Finite fin(qx[0]);
-        fin.add(qy[0]);
-        fin.add(qx[1]);
-        fin.add(qy[1]);
-        fin.add(qx[2]);
-        fin.add(qy[2]);
-        if (__builtin_expect(!(exact && n.ok() && fin.ok()), 0)) {
+        if (__builtin_expect(!(exact && n.ok() && big.ok()), 0)) {
 #pragma unroll
             for (int v = 0; v < 3; ++v) { qx[v] = sx[v] / area; qy[v] = sy[v] / area; }
         }
